@@ -542,18 +542,16 @@ static hk_status opacity_sectioned(hk_ctx *c, int nstates, bool mixed, int shape
     }
     for (const Sec &q : secs) {
       const LinesDev Ls = lines_sub(c->L, q.L0, q.L1 - q.L0);
-      const VoigtPlan plan = plan_voigt_section(mixed, shape, nx, q.t0, q.t1 - q.t0, 0);
-      if (plan.nsplit > 1) {
-        CUDA_TRY(c, c->vpart.ensure(plan.partial_doubles * sizeof(double)));
-        CUDA_TRY(c, c->vcnt.ensure(plan.counters * sizeof(unsigned)));
-      }
+      const VoigtPlan plan = plan_voigt_section(mixed, shape, c->g, n, q.t0, q.t1 - q.t0, 0);
+      if (plan.nsplit > 1) CUDA_TRY(c, c->vpart.ensure(plan.partial_doubles * sizeof(double)));
+      CUDA_TRY(c, c->vcnt.ensure(plan.work_bytes));
       CUDA_TRY(c, launch_line_records(mixed, Ls, c->g, sd + st, c->prep.p, s));
       CUDA_TRY(c, cudaEventRecord(c->ev[0], s));
-      CUDA_TRY(c, launch_voigt_sum(mixed, plan, c->prep.p, Ls.nu0, Ls.n, c->g, sd + st,
+      CUDA_TRY(c, launch_voigt_sum(mixed, plan, c->prep.p, Ls.nu0, Ls.n, c->g, sd + st, nullptr,
                                    c->ticket.as<unsigned>(), c->vpart.as<double>(),
-                                   c->vcnt.as<unsigned>(), Kd + (size_t)st * nx, nx, s));
+                                   c->vcnt.p, Kd + (size_t)st * nx, nx, s));
       CUDA_TRY(c, cudaEventRecord(c->ev[1], s));
-      c->launches += 2;
+      c->launches += 3;
       float ms = 0.f;
       CUDA_TRY(c, cudaEventSynchronize(c->ev[1]));
       CUDA_TRY(c, cudaEventElapsedTime(&ms, c->ev[0], c->ev[1]));
@@ -603,7 +601,7 @@ static hk_status tune_shape(hk_ctx *c, int nstates, const std::vector<StateDev> 
   int np = std::max(1, std::min({4, nstates / 12, (int)std::min<size_t>(4, c->prep_budget / per_state)}));
   const int G0 = voigt_tile_points(0);  // the widest tile; every shape's tile divides it
   const int tps0 = (int)((nx + G0 - 1) / G0);
-  const VoigtPlan p0 = plan_voigt_sum(true, 0, nx, 1, 0);
+  const VoigtPlan p0 = plan_voigt_sum(true, 0, c->g, n, 1, 0);
   const int sec = std::min(tps0, std::max((tps0 + 3) / 4, (2 * p0.ctas + p0.nsplit - 1) / p0.nsplit));
   const int first = (tps0 - sec) / 2;
   const int64_t x0 = (int64_t)first * G0, x1 = std::min<int64_t>((int64_t)(first + sec) * G0, nx);
@@ -619,27 +617,25 @@ static hk_status tune_shape(hk_ctx *c, int nstates, const std::vector<StateDev> 
   unsigned long long *twb = reinterpret_cast<unsigned long long *>(tsd + np);
   CUDA_TRY(c, cudaMemcpyAsync(tsd, ps.data(), np * sizeof(StateDev), cudaMemcpyHostToDevice, s));
   CUDA_TRY(c, c->prep.ensure((size_t)np * per_state));
-  CUDA_TRY(c, launch_line_prep(true, c->L, c->g, tsd, np, c->prep.p, twb, s));
+  CUDA_TRY(c, launch_line_prep(true, c->L, c->g, tsd, np, c->prep.p, twb, true, s));
   c->launches += 2;
   c->tune_ms.assign(nsh, -1.0);
   int best = 0;
   for (int v = 0; v < nsh; ++v) {
     const int G = voigt_tile_points(v);
     const int t0 = (int)(x0 / G), nt = (int)((x1 - x0 + G - 1) / G);
-    const VoigtPlan pw = plan_voigt_section(true, v, nx, t0, 1, 0);
-    const VoigtPlan pl = plan_voigt_section(true, v, nx, t0, nt, pw.ctas);
-    if (pl.nsplit > 1) {
-      CUDA_TRY(c, c->vpart.ensure(pl.partial_doubles * sizeof(double)));
-      CUDA_TRY(c, c->vcnt.ensure(pl.counters * sizeof(unsigned)));
-    }
-    CUDA_TRY(c, launch_voigt_sum(true, pw, c->prep.p, c->L.nu0, n, c->g, tsd, c->ticket.as<unsigned>(),
-                                 c->vpart.as<double>(), c->vcnt.as<unsigned>(), Kd, nx, s));
+    const VoigtPlan pw = plan_voigt_section(true, v, c->g, n, t0, 1, 0);
+    const VoigtPlan pl = plan_voigt_section(true, v, c->g, n, t0, nt, pw.ctas);
+    if (pl.nsplit > 1) CUDA_TRY(c, c->vpart.ensure(pl.partial_doubles * sizeof(double)));
+    CUDA_TRY(c, c->vcnt.ensure(pl.work_bytes));
+    CUDA_TRY(c, launch_voigt_sum(true, pw, c->prep.p, c->L.nu0, n, c->g, tsd, nullptr, c->ticket.as<unsigned>(),
+                                 c->vpart.as<double>(), c->vcnt.p, Kd, nx, s));
     double ms_v = 0.0;
     for (int k = 0; k < np; ++k) {
       const char *pk = static_cast<const char *>(c->prep.p) + (size_t)k * per_state;
       CUDA_TRY(c, cudaEventRecord(c->ev[0], s));
-      CUDA_TRY(c, launch_voigt_sum(true, pl, pk, c->L.nu0, n, c->g, tsd + k, c->ticket.as<unsigned>(),
-                                   c->vpart.as<double>(), c->vcnt.as<unsigned>(), Kd + (size_t)k * nx,
+      CUDA_TRY(c, launch_voigt_sum(true, pl, pk, c->L.nu0, n, c->g, tsd + k, nullptr, c->ticket.as<unsigned>(),
+                                   c->vpart.as<double>(), c->vcnt.p, Kd + (size_t)k * nx,
                                    nx, s));
       CUDA_TRY(c, cudaEventRecord(c->ev[1], s));
       CUDA_TRY(c, cudaEventSynchronize(c->ev[1]));
@@ -647,7 +643,7 @@ static hk_status tune_shape(hk_ctx *c, int nstates, const std::vector<StateDev> 
       CUDA_TRY(c, cudaEventElapsedTime(&ms, c->ev[0], c->ev[1]));
       ms_v += ms;
     }
-    c->launches += 1 + np;
+    c->launches += 2 * (1 + np);
     c->tune_ms[v] = ms_v;
     c->voigt_ms_acc += ms_v;  // probe sweeps count as line-sum time
     if (v == 0 || ms_v < c->tune_ms[best]) best = v;  // ties keep the lower shape
@@ -752,7 +748,7 @@ hk_status hk_opacity(hk_ctx *c, int nstates, const double *T, const double *P, i
   const int shape = shape_for(c, mixed);
   c->last_shape = shape;
   int batch = (int)std::max<size_t>(1, c->prep_budget / per_state);
-  const int nsplit = voigt_nsplit(nx, shape);
+  const int nsplit = voigt_nsplit(c->g, c->nlines, shape);
   if (nsplit > 1) {
     // split tiles keep one partial row per part: bound that scratch too
     const int G = voigt_tile_points(shape);
@@ -770,17 +766,15 @@ hk_status hk_opacity(hk_ctx *c, int nstates, const double *T, const double *P, i
   unsigned long long *wb = c->wbits.as<unsigned long long>();
   for (int b0 = 0; per_state <= c->prep_budget && b0 < nstates; b0 += batch) {
     const int nb = std::min(batch, nstates - b0);
-    const VoigtPlan plan = plan_voigt_sum(mixed, shape, nx, nb, 0);
-    c->launches += 3;  // line prep, state finalize, Voigt sum
-    if (plan.nsplit > 1) {
-      CUDA_TRY(c, c->vpart.ensure(plan.partial_doubles * sizeof(double)));
-      CUDA_TRY(c, c->vcnt.ensure(plan.counters * sizeof(unsigned)));
-    }
-    CUDA_TRY(c, launch_line_prep(mixed, c->L, c->g, sd + b0, nb, c->prep.p, wb + 2 * b0, s));
+    const VoigtPlan plan = plan_voigt_sum(mixed, shape, c->g, c->nlines, nb, 0);
+    c->launches += 3;  // line prep, state scale and tile ranges, Voigt sum
+    if (plan.nsplit > 1) CUDA_TRY(c, c->vpart.ensure(plan.partial_doubles * sizeof(double)));
+    CUDA_TRY(c, c->vcnt.ensure(plan.work_bytes));
+    CUDA_TRY(c, launch_line_prep(mixed, c->L, c->g, sd + b0, nb, c->prep.p, wb + 2 * b0, false, s));
     CUDA_TRY(c, cudaEventRecord(c->ev[0], s));
     CUDA_TRY(c, launch_voigt_sum(mixed, plan, c->prep.p, c->L.nu0, c->nlines, c->g,
-                                 sd + b0, c->ticket.as<unsigned>(), c->vpart.as<double>(),
-                                 c->vcnt.as<unsigned>(), Kd + (size_t)b0 * nx, nx, s));
+                                 sd + b0, wb + 2 * b0, c->ticket.as<unsigned>(), c->vpart.as<double>(),
+                                 c->vcnt.p, Kd + (size_t)b0 * nx, nx, s));
     CUDA_TRY(c, cudaEventRecord(c->ev[1], s));
     c->have_voigt_t = true;
     if (b0 + nb < nstates) {
@@ -1127,7 +1121,7 @@ static hk_status opacity_vjp(hk_ctx *c, double T, double P, int precision, const
   CUDA_TRY(c, c->prep.ensure((size_t)std::max<int64_t>(n, 1) * sizeof(LinePrep)));
   // the plain per-line records (FP64 windows and constants) of this state
   CUDA_TRY(c, launch_line_prep(false, c->L, c->g, c->states.as<StateDev>(), 1, c->prep.p,
-                               c->wbits.as<unsigned long long>(), s));
+                               c->wbits.as<unsigned long long>(), true, s));
   // the device copy of the state (wmax finalised) drives both passes
   CUDA_TRY(c, cudaMemcpyAsync(hs.data(), c->states.p, sizeof(StateDev), cudaMemcpyDeviceToHost, s));
   CUDA_TRY(c, cudaStreamSynchronize(s));
@@ -1211,7 +1205,7 @@ static hk_status table_build_batched(hk_ctx *c, int nstates, bool mixed, int sha
     return fail(c, HK_ERR_UNSUPPORTED, "one state's line records (%zu B) exceed the workspace (%zu B): "
                 "tables of such lists run through hk_opacity's sectioned path", per_state, c->prep_budget);
   int batch = (int)std::max<size_t>(1, c->prep_budget / per_state);
-  const int nsplit = voigt_nsplit(nx, shape);
+  const int nsplit = voigt_nsplit(c->g, c->nlines, shape);
   if (nsplit > 1) {
     const int G = voigt_tile_points(shape);
     const size_t part_per_state = (size_t)((nx + G - 1) / G) * nsplit * G * sizeof(double);
@@ -1219,11 +1213,9 @@ static hk_status table_build_batched(hk_ctx *c, int nstates, bool mixed, int sha
   }
   batch = std::min(batch, nstates);
   CUDA_TRY(c, c->prep.ensure((size_t)batch * per_state));
-  const VoigtPlan plan0 = plan_voigt_sum(mixed, shape, nx, batch, 0);
-  if (plan0.nsplit > 1) {
-    CUDA_TRY(c, c->vpart.ensure(plan0.partial_doubles * sizeof(double)));
-    CUDA_TRY(c, c->vcnt.ensure(plan0.counters * sizeof(unsigned)));
-  }
+  const VoigtPlan plan0 = plan_voigt_sum(mixed, shape, c->g, c->nlines, batch, 0);
+  if (plan0.nsplit > 1) CUDA_TRY(c, c->vpart.ensure(plan0.partial_doubles * sizeof(double)));
+  CUDA_TRY(c, c->vcnt.ensure(plan0.work_bytes));
   hk_status st;
   if ((st = ensure_qr(c, nC, 0)) != HK_OK) return st;
   const size_t nscr = kdist_scratch_doubles(c->nxb, c->nbins, nstates);
@@ -1239,13 +1231,13 @@ static hk_status table_build_batched(hk_ctx *c, int nstates, bool mixed, int sha
   int64_t kernels = 0;
   for (int b0 = 0; e == cudaSuccess && b0 < nstates; b0 += batch) {
     const int nb = std::min(batch, nstates - b0);
-    const VoigtPlan plan = plan_voigt_sum(mixed, shape, nx, nb, plan0.ctas);
-    e = launch_line_prep(mixed, c->L, c->g, sd + b0, nb, c->prep.p, wb + 2 * b0, cs);
+    const VoigtPlan plan = plan_voigt_sum(mixed, shape, c->g, c->nlines, nb, plan0.ctas);
+    e = launch_line_prep(mixed, c->L, c->g, sd + b0, nb, c->prep.p, wb + 2 * b0, false, cs);
     if (e == cudaSuccess)
-      e = launch_voigt_sum(mixed, plan, c->prep.p, c->L.nu0, c->nlines, c->g, sd + b0,
-                           c->ticket.as<unsigned>(), c->vpart.as<double>(), c->vcnt.as<unsigned>(),
+      e = launch_voigt_sum(mixed, plan, c->prep.p, c->L.nu0, c->nlines, c->g, sd + b0, wb + 2 * b0,
+                           c->ticket.as<unsigned>(), c->vpart.as<double>(), c->vcnt.p,
                            K + (size_t)b0 * nx, nx, cs);
-    kernels += 3;  // line prep, state scale, Voigt sum
+    kernels += 3;  // line prep, state scale and tile ranges, Voigt sum
   }
   if (e == cudaSuccess) {
     e = launch_kdist(K, nx, nstates, c->nxb, c->nbins, nC, c->kmin, unitScale, c->qrV.as<double>(),
@@ -1312,7 +1304,7 @@ hk_status hk_table_build(hk_ctx *c, int nstates, const double *T, const double *
     return table_build_batched(c, nstates, mixed, shape, K, nC, unitScale, coeff, nxmin);
   // one persistent launch for the whole table: line prep into a ring of
   // per-state record slots and every state's Voigt sums (hkb_voigt.cu)
-  const TablePlan tp = plan_table(mixed, shape, c->nlines, nx, nstates);
+  const TablePlan tp = plan_table(mixed, shape, c->nlines, c->g, nstates);
   if (tp.ring_bytes > c->prep_budget)
     return fail(c, HK_ERR_UNSUPPORTED, "%d states' line records (%zu B) exceed the workspace (%zu B): "
                 "tables of such lists run through hk_opacity's sectioned path", tp.slots, tp.ring_bytes,

@@ -33,9 +33,11 @@ cudaError_t launch_opacity_vjp(bool mixed, const LinesDev &L, const GridDev &g,
                                double *G_d, const int64_t *order_d, double *dlogS_d,
                                double *dgam_d, int log_gamma, double *dTP_d, cudaStream_t stream);
 
-// per-(line, state) records: LinePrepF (mixed) or LinePrep (plain FP64)
+// per-(line, state) records: LinePrepF (mixed) or LinePrep (plain FP64), and
+// the states' maxima (wbits_d, two words each); scale: also the states' cutoff
+// bound and FP32 scale from them (else launch_voigt_sum forms them)
 cudaError_t launch_line_prep(bool mixed, const LinesDev &L, const GridDev &g, StateDev *states_d,
-                             int nstates, void *prep_d, unsigned long long *wbits_d,
+                             int nstates, void *prep_d, unsigned long long *wbits_d, bool scale,
                              cudaStream_t stream);
 // Sectioned states (a state's records larger than the workspace): the state
 // pass (cutoff bound, FP32 scale) over all lines, then one section's records
@@ -127,17 +129,21 @@ struct VoigtPlan {
   int nsplit = 1;
   size_t partial_doubles = 0;
   size_t counters = 0;
+  size_t work_bytes = 0;  // the tiles' line ranges and counters
 };
-VoigtPlan plan_voigt_sum(bool mixed, int shape, int64_t nx, int nstates, int grid_ctas);
+VoigtPlan plan_voigt_sum(bool mixed, int shape, const GridDev &g, int64_t nlines, int nstates,
+                         int grid_ctas);
 // tiles [tile0, tile0 + ntiles) of each state's grid
-VoigtPlan plan_voigt_section(bool mixed, int shape, int64_t nx, int tile0, int ntiles, int grid_ctas);
-// line-range parts per tile for a grid of nx points in tiles of the shape
-int voigt_nsplit(int64_t nx, int shape);
+VoigtPlan plan_voigt_section(bool mixed, int shape, const GridDev &g, int64_t nlines, int tile0,
+                             int ntiles, int grid_ctas, int nstates = 1);
+// line-range parts per tile for a grid in tiles of the shape and a list of
+// nlines lines (the whole list, also for a section's launch)
+int voigt_nsplit(const GridDev &g, int64_t nlines, int shape);
 cudaError_t launch_voigt_sum(bool mixed, const VoigtPlan &plan, const void *prep_d,
                              const double *nu0_d, int64_t nlines, const GridDev &g,
-                             const StateDev *states_d, unsigned *ticket_d, double *partial_d,
-                             unsigned *tile_cnt_d, double *K_d, int64_t k_stride,
-                             cudaStream_t stream);
+                             StateDev *states_d, const unsigned long long *wbits_d,
+                             unsigned *ticket_d, double *partial_d, void *work_d, double *K_d,
+                             int64_t k_stride, cudaStream_t stream);
 
 // A whole T-P table as one persistent launch (hkb_voigt.cu): line prep into
 // a ring of per-state record slots and the Voigt sums of every state, as
@@ -170,7 +176,7 @@ inline size_t table_sync_bytes(int nstates) {
   // ticket (8) + pad (8), wbits 16 S, fin 16 S, prep/sum counts and ready flags 12 S, error word
   return 16 + 16 * (size_t)nstates + sizeof(TableFin) * (size_t)nstates + 12 * (size_t)nstates + 16;
 }
-TablePlan plan_table(bool mixed, int shape, int64_t nlines, int64_t nx, int nstates);
+TablePlan plan_table(bool mixed, int shape, int64_t nlines, const GridDev &g, int nstates);
 cudaError_t launch_voigt_table(bool mixed, const TablePlan &plan, const LinesDev &L, const GridDev &g,
                                const StateDev *states_d, const TableBufs &bufs, double *K_d,
                                int64_t k_stride, cudaStream_t stream);

@@ -135,10 +135,7 @@ __global__ void state_finalize_kernel(GridDev g, StateDev *__restrict__ states,
   double wmax;
   int e;
   state_scale(g, wbits[2 * s], wbits[2 * s + 1], wmax, e);
-  states[s].wmax = wmax;
-  states[s].s1scale = ldexp(1.0, e);
-  states[s].s1unscale = ldexp(1.0, -e);
-  states[s].s1exp = e;
+  put_state_scale(states[s], wmax, e);
 }
 
 // Exact (line, grid point) pair counts of one state by region, from the same
@@ -192,7 +189,7 @@ cudaError_t launch_count_pairs(const LinesDev &L, const GridDev &g, const StateD
 
 cudaError_t launch_line_prep(bool mixed, const LinesDev &L, const GridDev &g, StateDev *states_d,
                              int nstates, void *prep_d, unsigned long long *wbits_d,
-                             cudaStream_t stream) {
+                             bool scale, cudaStream_t stream) {
   cudaError_t e = cudaMemsetAsync(wbits_d, 0, 2 * nstates * sizeof(unsigned long long), stream);
   if (e != cudaSuccess) return e;
   if (L.n > 0) {
@@ -206,6 +203,7 @@ cudaError_t launch_line_prep(bool mixed, const LinesDev &L, const GridDev &g, St
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
+  if (!scale) return cudaSuccess;
   state_finalize_kernel<<<(nstates + 127) / 128, 128, 0, stream>>>(g, states_d, nstates, wbits_d);
   return cudaGetLastError();
 }

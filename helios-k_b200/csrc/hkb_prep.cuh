@@ -173,4 +173,11 @@ __device__ __forceinline__ void state_scale(const GridDev &g, unsigned long long
   s1exp = e;
 }
 
+__device__ __forceinline__ void put_state_scale(StateDev &st, double wmax, int e) {
+  st.wmax = wmax;
+  st.s1scale = ldexp(1.0, e);
+  st.s1unscale = ldexp(1.0, -e);
+  st.s1exp = e;
+}
+
 }  // namespace hkb

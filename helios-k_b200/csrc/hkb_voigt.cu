@@ -150,13 +150,13 @@ constexpr int HK_RPAD = 8;
 // Far field (the default option set): each warp's FP64 sums of the blocks'
 // Taylor coefficients, HK_FN per 64-point block.
 constexpr int HK_FB = 64, HK_FN = 9;
-template <class SH, int EXT = HK_EXT_NONE>
+template <class SH, int EXT = HK_EXT_NONE, int SUB = 1>
 constexpr size_t smem_mixed() {
   return sizeof(RecF) * SH::CH + sizeof(float) * (HK_RPAD + SH::CH * HK_C916_MR) +
-         sizeof(double) * SH::G +
+         sizeof(double) * (SH::G / SUB) +
          (EXT == HK_EXT_CHI ? sizeof(float) * SH::CH
           : EXT == HK_EXT_PL ? sizeof(ExtPL) * SH::CH
-                             : sizeof(double) * SH::WARPS * HK_FN * (SH::G / HK_FB));
+                             : sizeof(double) * SH::WARPS * HK_FN * (SH::G / SUB / HK_FB));
 }
 
 struct __align__(16) RecD {
@@ -1075,58 +1075,69 @@ __device__ __forceinline__ void flush_sums(float2 (&a32)[PPL / 2], double *__res
   for (int q = 0; q < PPL / 2; ++q) a32[q] = make_float2(0.f, 0.f);
 }
 
+// The nu-sorted lines whose windows can reach grid points [g0, g1), wmax the
+// state's search half-width and shift its largest pressure shift: the first
+// (end = false) or past the last; all 32
+// lanes call it.
+__device__ __forceinline__ int64_t tile_lines(const double *__restrict__ nu0, int64_t nlines,
+                                              const GridDev &g, double shift, double wmax,
+                                              int64_t g0, int64_t g1, bool end) {
+  const double W = wmax + shift + 2.0 * g.dnu;
+  const double xlo = grid_x(g, g0) - W;
+  const double xhi = grid_x(g, g1 - 1) + W;
+  const double pad = 1e-12 * (fabs(xlo) + fabs(xhi)) + 1e-300;
+  return lower_bound_warp(nu0, nlines, end ? xhi + pad : xlo - pad);
+}
+
 // ------------------------------------------------------- one tile's sum
 // Everything one ticket of the Voigt sum does: the sum of the lines whose
 // windows reach the tile [g0, g1) (the part-th of nsplit parts of its line
 // range) into the tile's points, written to Ks (one state's K row) or, for a
 // split tile, published to pt (this tile's nsplit partial rows of G points)
 // and combined in part order by the CTA that completes the count *cnt.
-// wmax and s1exp are the state's search half-width and FP32 scale exponent.
-template <bool MIXED, class SH, bool CG, bool G34 = false, int EXT = HK_EXT_NONE>
-__device__ __forceinline__ void sum_tile(const void *prep_s, const double *__restrict__ nu0,
-                                         int64_t nlines, const GridDev &g, const StateDev &st,
-                                         double wmax, int s1exp, int64_t g0, int64_t g1, int part,
+// [L0, L1) are the lines whose windows can reach the tile (tile_lines) and
+// s1exp the state's FP32 scale exponent.
+// SUB > 1: the CTA sums the sub-th of SUB equal parts of the tile's points
+// (SL points per warp instead of SLICE) with everything a point's sum depends
+// on -- the chunks, the classes of a line for the SLICE-point slice its points
+// lie in, the order of levels and classes, the far field's lines per warp --
+// as in the whole tile, so the sums are the same to the bit.  It stages and
+// classifies the lines SUB times over, and pays where a call has too few
+// tickets to fill the GPU (launch_voigt_sum).
+template <bool MIXED, class SH, bool CG, bool G34 = false, int EXT = HK_EXT_NONE, int SUB = 1>
+__device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t L1,
+                                         const GridDev &g, const StateDev &st, int s1exp, int64_t g0,
+                                         int64_t g1, int part,
                                          int nsplit, double *pt, unsigned *cnt, double *Ks,
-                                         unsigned char *smem_dyn) {
+                                         unsigned char *smem_dyn, int sub = 0) {
   using Rec = typename std::conditional<MIXED, RecF, RecD>::type;
-  constexpr int CH = SH::CH, PPL = SH::PPL, SLICE = SH::SLICE, G = SH::G;
+  constexpr int CH = SH::CH, PPL = SH::PPL / SUB, SLICE = SH::SLICE, G = SH::G;
+  constexpr int SL = SLICE / SUB, GS = G / SUB;  // points per warp and CTA
+  static_assert(SUB == 1 || (SL % HK_FB == 0 && PPL % 2 == 0 && EXT == HK_EXT_NONE && !G34), "sub-tiles");
   // the far field runs in the mixed form without options (Voigt, Lorentz)
   constexpr bool FAR = MIXED && !G34 && EXT == HK_EXT_NONE;
-  constexpr int NBLK = G / HK_FB;  // 64-point blocks of the tile (<= 32)
-  static_assert(!FAR || (NBLK <= 32 && SLICE % HK_FB == 0), "far-field block layout");
+  constexpr int NBLK = GS / HK_FB;  // 64-point blocks of the CTA's points
+  static_assert(!FAR || (G / HK_FB <= 32 && SL % HK_FB == 0), "far-field block layout");
   Rec *rec = reinterpret_cast<Rec *>(smem_dyn);
   float *Rtab = reinterpret_cast<float *>(smem_dyn + sizeof(Rec) * CH) + HK_RPAD;
   double *cacc = reinterpret_cast<double *>(smem_dyn + sizeof(Rec) * CH +
                                             sizeof(float) * (HK_RPAD + CH * HK_C916_MR));
   __shared__ int s_last;
   __shared__ int s_kcnt[CH / 32][HK_NKEY];  // staged lines per (staging warp, key)
-  __shared__ long long s_L0, s_L1;
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
-  const int wb = warp * SLICE;
+  const int wb = sub * GS + warp * SL;   // the warp's first tile point
+  const int ws = wb - wb % SLICE;        // the slice its lines are classed for
   const LinePrep *P = reinterpret_cast<const LinePrep *>(prep_s);
   const LinePrepF *PF = reinterpret_cast<const LinePrepF *>(prep_s);
-  if (warp == 0) {
-    const double W = wmax + st.shift + 2.0 * g.dnu;
-    const double xlo = grid_x(g, g0) - W;
-    const double xhi = grid_x(g, g1 - 1) + W;
-    const double pad = 1e-12 * (fabs(xlo) + fabs(xhi)) + 1e-300;
-    const int64_t L0 = lower_bound_warp(nu0, nlines, xlo - pad);
-    const int64_t L1 = lower_bound_warp(nu0, nlines, xhi + pad);
-    if (lane == 0) {
-      s_L0 = L0;
-      s_L1 = L1;
-    }
-  }
-  __syncthreads();
-  const int64_t L0 = s_L0, L1 = s_L1;
   // per staged line: 1 / nu (chi factor) or ExtPL (plinth), after the
   // per-point sums
-  float *ext_inu = reinterpret_cast<float *>(cacc + G);
-  ExtPL *ext_pl = reinterpret_cast<ExtPL *>(cacc + G);
+  float *ext_inu = reinterpret_cast<float *>(cacc + GS);
+  ExtPL *ext_pl = reinterpret_cast<ExtPL *>(cacc + GS);
   // far field: warp w's coefficient sums fd[(w HK_FN + n) NBLK + block]
-  double *fd = cacc + G;
+  double *fd = cacc + GS;
+  cacc -= sub * GS;  // indexed by tile point
   if (FAR)
     for (int t = lane; t < HK_FN * NBLK; t += 32) fd[warp * HK_FN * NBLK + t] = 0.0;
   ExtF exc;
@@ -1163,6 +1174,9 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, const double *__res
   // and leave the other warps idle at the barrier).
   const int64_t nL = L1 - L0;
   const int64_t nch = (nL + CH - 1) / CH;
+  // every part of the tile finds the same number of parts: no empty ones
+  nsplit = (int)min((int64_t)nsplit, max(nch, (int64_t)1));
+  if (part >= nsplit) return;
   const int64_t c_begin = nch * part / nsplit, c_end = nch * (part + 1) / nsplit;
   int lcur = 0;  // strength level held in a32 (warp-uniform)
   for (int64_t c = c_begin; c < c_end; ++c) {
@@ -1207,7 +1221,8 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, const double *__res
       for (int g32 = 0; g32 < cnt_c; g32 += 32) {
         const int j = g32 + lane;
         unsigned fm = 0u;  // the line's far blocks in this slice
-        const int cls = (j < cnt_c) ? classify<SLICE, FAR>(rf[j], wb, fm) : HK_CLS_SKIP;
+        const int cls = (j < cnt_c) ? classify<SLICE, FAR>(rf[j], ws, fm) : HK_CLS_SKIP;
+        if (SUB > 1) fm >>= (wb - ws) / HK_FB;  // the warp's own blocks
         const int lev = (j < cnt_c) ? (rf[j].flags >> 8) : 0;
         const unsigned bB = __ballot_sync(0xffffffffu, cls == HK_CLS_B);
         const unsigned bA = __ballot_sync(0xffffffffu, cls == HK_CLS_A);
@@ -1236,7 +1251,7 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, const double *__res
               mX &= mX - 1;
               const float inu = ext_inu[g32 + b];
               sweep_G<false, false, PPL, EXT>(rf[g32 + b], wb, lane, kf, a32, cacc, g.profile, &exc, inu);
-              sweep_C<SLICE, EXT>(rf[g32 + b], Rtab + (g32 + b) * HK_C916_MR, cacc, wb, lane, &exc, inu);
+              sweep_C<SL, EXT>(rf[g32 + b], Rtab + (g32 + b) * HK_C916_MR, cacc, wb, lane, &exc, inu);
             }
             continue;
           }
@@ -1250,7 +1265,7 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, const double *__res
               const ExtPL *pe = ext_pl + g32 + b;
               sweep_G<false, false, PPL, EXT>(rf[g32 + b], wb, lane, kf, a32, cacc, g.profile, nullptr, 0.f,
                                               pe);
-              sweep_C<SLICE, EXT>(rf[g32 + b], Rtab + (g32 + b) * HK_C916_MR, cacc, wb, lane, nullptr, 0.f,
+              sweep_C<SL, EXT>(rf[g32 + b], Rtab + (g32 + b) * HK_C916_MR, cacc, wb, lane, nullptr, 0.f,
                                   (double)pe->plf * u);
             }
             continue;
@@ -1286,7 +1301,7 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, const double *__res
             mBM &= mBM - 1;
             const unsigned fb = FAR ? __shfl_sync(0xffffffffu, fm, b) : 0u;
             sweep_BM<PPL>(rf[g32 + b], wb, lane, kf, a32, fb);
-            sweep_C<SLICE>(rf[g32 + b], Rtab + (g32 + b) * HK_C916_MR, cacc, wb, lane);
+            sweep_C<SL>(rf[g32 + b], Rtab + (g32 + b) * HK_C916_MR, cacc, wb, lane);
           }
           while (mAM) {
             const int b = __ffs(mAM) - 1;
@@ -1303,7 +1318,7 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, const double *__res
             mG &= mG - 1;
             const unsigned fb = FAR ? __shfl_sync(0xffffffffu, fm, b) : 0u;
             sweep_G<false, G34, PPL>(rf[g32 + b], wb, lane, kf, a32, cacc, g.profile, nullptr, 0.f, nullptr, fb);
-            sweep_C<SLICE>(rf[g32 + b], Rtab + (g32 + b) * HK_C916_MR, cacc, wb, lane);
+            sweep_C<SL>(rf[g32 + b], Rtab + (g32 + b) * HK_C916_MR, cacc, wb, lane);
           }
         }
         while (mW) {
@@ -1312,7 +1327,7 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, const double *__res
           if (EXT == HK_EXT_CHI && chi_tile) {
             const float inu = ext_inu[g32 + b];
             sweep_G<true, false, PPL, EXT>(rf[g32 + b], wb, lane, kf, a32, cacc, g.profile, &exc, inu);
-            sweep_C<SLICE, EXT>(rf[g32 + b], Rtab + (g32 + b) * HK_C916_MR, cacc, wb, lane, &exc, inu);
+            sweep_C<SL, EXT>(rf[g32 + b], Rtab + (g32 + b) * HK_C916_MR, cacc, wb, lane, &exc, inu);
           } else if constexpr (EXT == HK_EXT_PL) {
             // FP64 sums (S1f = 1): the plinth per S1 scaled by S1, or the
             // whole line per point in FP64
@@ -1324,12 +1339,12 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, const double *__res
               sweep_pl64<PPL>(rw, *pe, wb, lane, cacc, g.profile);
             } else {
               sweep_G<true, false, PPL, EXT>(rw, wb, lane, kf, a32, cacc, g.profile, nullptr, 0.f, pe);
-              sweep_C<SLICE, EXT>(rw, Rtab + (g32 + b) * HK_C916_MR, cacc, wb, lane, nullptr, 0.f,
+              sweep_C<SL, EXT>(rw, Rtab + (g32 + b) * HK_C916_MR, cacc, wb, lane, nullptr, 0.f,
                                   (double)pe->plf * (rw.Sc * (double)rw.y * 0.56418958354775628));
             }
           } else {
             sweep_G<true, G34, PPL>(rf[g32 + b], wb, lane, kf, a32, cacc, g.profile);
-            sweep_C<SLICE>(rf[g32 + b], Rtab + (g32 + b) * HK_C916_MR, cacc, wb, lane);
+            sweep_C<SL>(rf[g32 + b], Rtab + (g32 + b) * HK_C916_MR, cacc, wb, lane);
           }
         }
       }
@@ -1338,7 +1353,8 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, const double *__res
       if constexpr (FAR) {
         // far field: warp w takes lines w, w + WARPS, ... (strength-level
         // order), lane = block of the tile
-        const int blo = lane * HK_FB;
+        const int fb0 = sub * NBLK;  // the CTA's first block in the tile
+        const int blo = (fb0 + lane) * HK_FB;
         double *fdw = fd + warp * HK_FN * NBLK;
         float fq[HK_FN];
 #pragma unroll
@@ -1348,7 +1364,7 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, const double *__res
           const RecF &r = rf[j];
           const unsigned fmk = r.fmask;
           if (fmk == 0u) continue;
-          const bool far = (fmk >> lane) & 1u;
+          const bool far = SUB == 1 ? (fmk >> lane) & 1u : lane < NBLK && ((fmk >> (fb0 + lane)) & 1u);
           const int lev = r.flags >> 8;
           if (lev != flev) {
             if (flev >= 0) far_flush(fq, fdw, lane, NBLK, s1exp, flev);
@@ -1378,8 +1394,8 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, const double *__res
 #pragma unroll
     for (int p = 0; p < PPL; ++p) {
       const int k = wb + lane + 32 * p;
-      const int bl = k / HK_FB;
-      const double jj = (double)(k - bl * HK_FB) - 31.5;
+      const int bl = (k - sub * GS) / HK_FB;
+      const double jj = (double)(k % HK_FB) - 31.5;
       double v = fd[(HK_FN - 1) * NBLK + bl];
 #pragma unroll
       for (int n = HK_FN - 2; n >= 0; --n) v = fma(v, jj, fd[n * NBLK + bl]);
@@ -1411,26 +1427,64 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, const double *__res
     __syncthreads();
     if (s_last) {
       __threadfence();
+      // (the parts in the outer loop: PPL independent loads in flight)
+#pragma unroll
+      for (int p = 0; p < PPL; ++p) acc[p] = 0.0;
+#pragma unroll 2
+      for (int j = 0; j < nsplit; ++j) {
+        const double *pj = pt + (int64_t)j * G + wb + lane;
+#pragma unroll
+        for (int p = 0; p < PPL; ++p) acc[p] += __ldcg(pj + 32 * p);
+      }
 #pragma unroll
       for (int p = 0; p < PPL; ++p) {
-        const int k = wb + lane + 32 * p;
-        double sum = 0.0;
-        for (int j = 0; j < nsplit; ++j) sum += __ldcg(pt + (int64_t)j * G + k);
-        const int64_t gi = g0 + k;
-        if (gi < g1) Ks[gi] = st.kmin + sum;
+        const int64_t gi = g0 + wb + lane + 32 * p;
+        if (gi < g1) Ks[gi] = st.kmin + acc[p];
       }
       if (tid == 0) atomicExch(cnt, 0u);
     }
   }
 }
 
+// The line range of every tile of a launch (a warp per range end), the scale
+// of its states from the line prep's maxima (wbits; null: the states hold it)
+// and the launch's ticket and tile counters from zero.  A ticket that searched
+// for its own lines spent ~4 us of dependent loads on it, a tenth of a small
+// state's part; this launch takes the place of the state scale's and of two
+// memsets.
+__global__ void __launch_bounds__(256)
+tile_range_kernel(const double *__restrict__ nu0, int64_t nlines, GridDev g,
+                  StateDev *states, const unsigned long long *__restrict__ wbits, int G, int tile0,
+                  int tiles_per_state, int64_t tiles, int64_t *__restrict__ ranges, unsigned *__restrict__ ticket,
+                  unsigned *__restrict__ tile_cnt, int64_t ncnt) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == 0) *ticket = 0u;
+  for (int64_t i = t; i < ncnt; i += (int64_t)gridDim.x * blockDim.x) tile_cnt[i] = 0u;
+  const int64_t w = t >> 5;
+  if (w >= 2 * tiles) return;
+  const int64_t tt = w >> 1;
+  const int s = (int)(tt / tiles_per_state);
+  const int64_t tile = tt - (int64_t)s * tiles_per_state, g0 = (tile0 + tile) * G;
+  StateDev &st = states[s];
+  double wmax;
+  if (wbits) {
+    int e;
+    state_scale(g, wbits[2 * s], wbits[2 * s + 1], wmax, e);
+    if (tile == 0 && (threadIdx.x & 31) == 0 && !(w & 1)) put_state_scale(st, wmax, e);
+  } else {
+    wmax = st.wmax;
+  }
+  const int64_t v = tile_lines(nu0, nlines, g, st.shift, wmax, g0, min(g0 + (int64_t)G, g.nx), w & 1);
+  if ((threadIdx.x & 31) == 0) ranges[w] = v;
+}
+
 // ------------------------------------------------------- persistent kernel
 // mixed form: SH::MINB CTAs per SM (4: 32 warps, 64 registers)
 // G34: the Doppler / binned-Gaussian profiles of the mixed form (their own
 // instantiation, so the Voigt and Lorentz kernels carry none of their code)
-template <bool MIXED, class SH, bool G34 = false, int EXT = HK_EXT_NONE>
+template <bool MIXED, class SH, bool G34 = false, int EXT = HK_EXT_NONE, int SUB = 1>
 __global__ void __launch_bounds__(SH::THREADS, MIXED ? SH::MINB : 2)
-voigt_sum_kernel(const void *__restrict__ prep, const double *__restrict__ nu0,
+voigt_sum_kernel(const void *__restrict__ prep, const longlong2 *__restrict__ ranges,
                  int64_t nlines, GridDev g, const StateDev *__restrict__ states,
                  int tile0, int tiles_per_state, int nsplit, int total_tickets,
                  unsigned *__restrict__ ticket, double *__restrict__ partial,
@@ -1445,18 +1499,21 @@ voigt_sum_kernel(const void *__restrict__ prep, const double *__restrict__ nu0,
     __syncthreads();
     const int t = s_ticket;
     if (t >= total_tickets) break;
-    // ticket -> (tile of a state, part of that tile's line range)
-    const int tt = t / nsplit;
-    const int part = t - tt * nsplit;
+    // ticket -> (tile of a state, part of that tile's line range, sub-tile)
+    const int tp = t / SUB, sub = t - tp * SUB;
+    const int tt = tp / nsplit;
+    const int part = tp - tt * nsplit;
     const int s = tt / tiles_per_state;
     const int tile = tt - s * tiles_per_state;
     const StateDev &st = states[s];
     const void *prep_s = static_cast<const char *>(prep) + (size_t)s * nlines * rec_bytes;
     const int64_t g0 = (int64_t)(tile0 + tile) * G;
     const int64_t g1 = min(g0 + (int64_t)G, g.nx);
-    sum_tile<MIXED, SH, false, G34, EXT>(prep_s, nu0, nlines, g, st, st.wmax, st.s1exp, g0, g1, part, nsplit,
-                               partial + (int64_t)tt * nsplit * G, tile_cnt + tt,
-                               K + (int64_t)s * k_stride, smem_dyn);
+    const longlong2 L = ranges[tt];
+    sum_tile<MIXED, SH, false, G34, EXT, SUB>(prep_s, L.x, L.y, g, st, st.s1exp, g0, g1, part,
+                                              nsplit, partial + (int64_t)tt * nsplit * G,
+                                              tile_cnt + (int64_t)tt * SUB + sub,
+                                              K + (int64_t)s * k_stride, smem_dyn, sub);
   }
 }
 
@@ -1562,7 +1619,7 @@ voigt_table_kernel(LinesDev L, GridDev g, const StateDev *__restrict__ states, T
                    int64_t k_stride) {
   constexpr int G = SH::G, THREADS = SH::THREADS;
   extern __shared__ __align__(16) unsigned char smem_dyn[];
-  __shared__ long long s_ticket;
+  __shared__ long long s_ticket, s_range[2];
   __shared__ int s_go;
   __shared__ double s_e916[HK_SIG1_M];
   const int tid = threadIdx.x;
@@ -1623,7 +1680,12 @@ voigt_table_kernel(LinesDev L, GridDev g, const StateDev *__restrict__ states, T
         const int64_t g0 = (int64_t)tile * G;
         const int64_t g1 = min(g0 + (int64_t)G, g.nx);
         const size_t tslot = (size_t)slot * sc.tps + tile;
-        sum_tile<MIXED, SH, true, G34, EXT>(ring_s, L.nu0, n, g, st, f.wmax, f.s1exp, g0, g1, part, sc.nsplit,
+        if (tid < 64) {
+          const int64_t v = tile_lines(L.nu0, n, g, st.shift, f.wmax, g0, g1, tid >= 32);
+          if ((tid & 31) == 0) s_range[tid >> 5] = v;
+        }
+        __syncthreads();
+        sum_tile<MIXED, SH, true, G34, EXT>(ring_s, s_range[0], s_range[1], g, st, f.s1exp, g0, g1, part, sc.nsplit,
                                   partial + tslot * sc.nsplit * G, tile_cnt + tslot,
                                   K + (int64_t)s * k_stride, smem_dyn);
       }
@@ -1717,12 +1779,28 @@ static int ext_kind(const GridDev &g) {
   return HK_EXT_NONE;
 }
 
+// Sub-tiles (sum_tile's SUB) of the default shape, in both precisions.
+constexpr int HK_MAX_SUB = 4;
+
 // Calls f(kernel, dynamic shared memory) for the kernel of (precision,
-// shape); the plain FP64 form has the default shape only.
+// shape, sub-tiles); the plain FP64 form has the default shape only.
 template <class F>
-static cudaError_t with_kernel(bool mixed, int shape, F &&f, bool g34 = false, int ext = HK_EXT_NONE) {
-  using KFn = void (*)(const void *, const double *, int64_t, GridDev, const StateDev *, int, int,
+static cudaError_t with_kernel(bool mixed, int shape, F &&f, bool g34 = false, int ext = HK_EXT_NONE,
+                               int sub = 1) {
+  using KFn = void (*)(const void *, const longlong2 *, int64_t, GridDev, const StateDev *, int, int,
                        int, int, unsigned *, double *, unsigned *, double *, int64_t);
+#define HK_SUB_CASE(n)                                                                                \
+  case n:                                                                                             \
+    return mixed ? f((KFn)voigt_sum_kernel<true, Shape0, false, HK_EXT_NONE, n>,                      \
+                     smem_mixed<Shape0, HK_EXT_NONE, n>(), Shape0::THREADS)                           \
+                 : f((KFn)voigt_sum_kernel<false, Shape0, false, HK_EXT_NONE, n>,                     \
+                     sizeof(RecD) * Shape0::CH, Shape0::THREADS);
+  switch (sub) {
+    HK_SUB_CASE(2)
+    HK_SUB_CASE(HK_MAX_SUB)
+    default: break;
+  }
+#undef HK_SUB_CASE
   if (!mixed) return f((KFn)voigt_sum_kernel<false, Shape0>, sizeof(RecD) * Shape0::CH, Shape0::THREADS);
   if (g34 && ext == HK_EXT_PL)
     return f((KFn)voigt_sum_kernel<true, Shape0, true, HK_EXT_PL>, smem_mixed<Shape0, HK_EXT_PL>(),
@@ -1763,75 +1841,105 @@ static int voigt_ctas(bool mixed, int shape) {
 
 // Tiles are split along their line range when a state has few tiles: one
 // tile's sweep lasts ~1/3 of a 1e7-line state, so an unsplit 1465-tile grid
-// ends in a last wave that leaves most of the GPU idle for that long.  The
-// split depends on the grid and the tile shape only (HK_TICKETS_PER_STATE,
-// about 8 tickets per resident CTA of a 148-SM B200 at 4 CTAs/SM), never on
-// the batch or the device, so one state's K is bit-identical however it is
-// batched.
-constexpr int HK_TICKETS_PER_STATE = 4736;
-constexpr int HK_MAX_SPLIT = 8;
+// ends in a last wave that leaves most of the GPU idle for that long.  Up to
+// HK_SPLIT parts aim at HK_TICKETS_PER_STATE tickets, about 8 per resident
+// CTA of a 148-SM B200 at 4 CTAs/SM; a grid too small for that (8 parts of
+// fewer than 148 tiles) takes as many parts as give HK_TICKETS_SMALL, two per
+// resident CTA, at most HK_MAX_SPLIT and one per chunk of lines that a tile
+// holds (about).  1e5 lines on 2e4 points (10 tiles): 1.03 ms in 8 parts,
+// 0.34 ms in 64; 3e4 lines on 5e4 points 0.20 -> 0.13 ms, 24 states of it in
+// one launch 1.76 -> 1.67 ms.  The split depends on the grid, the line list
+// and the tile shape only, never on the batch or the device, so one state's K
+// is bit-identical however it is batched.
+constexpr int HK_TICKETS_PER_STATE = 4736, HK_TICKETS_SMALL = 1184;
+constexpr int HK_SPLIT = 8, HK_MAX_SPLIT = 64;
 
-int voigt_nsplit(int64_t nx, int shape) {
-  const int G = voigt_tile_points(shape);
-  const int64_t tps = (nx + G - 1) / G;
-  if (tps <= 0) return 1;
-  return (int)std::min<int64_t>(HK_MAX_SPLIT,
-                                std::max<int64_t>(1, (HK_TICKETS_PER_STATE + tps - 1) / tps));
+// A tile's chunks of lines, about: the lines spread over the grid, each
+// reaching its cut window (of a fixed width; else the tile alone) and the tile.
+static int64_t tile_chunks(const GridDev &g, int64_t nlines, int shape) {
+  const double reach = g.cutMode == 0 ? 2.0 * g.cut : 0.0, tile = voigt_tile_points(shape) * g.dnu;
+  const double nL = (double)nlines * std::min(1.0, (reach + tile) / (reach + (double)g.nx * g.dnu));
+  return (int64_t)(nL / voigt_chunk_lines(shape)) + 1;
 }
 
-VoigtPlan plan_voigt_section(bool mixed, int shape, int64_t nx, int tile0, int ntiles, int grid_ctas) {
+int voigt_nsplit(const GridDev &g, int64_t nlines, int shape) {
+  const int G = voigt_tile_points(shape);
+  const int64_t tps = (g.nx + G - 1) / G;
+  if (tps <= 0) return 1;
+  auto parts = [tps](int64_t tickets, int64_t most) {
+    return std::min<int64_t>(most, std::max<int64_t>(1, (tickets + tps - 1) / tps));
+  };
+  const int64_t most = std::min<int64_t>(HK_MAX_SPLIT, tile_chunks(g, nlines, shape));
+  return (int)std::max(parts(HK_TICKETS_PER_STATE, HK_SPLIT), parts(HK_TICKETS_SMALL, most));
+}
+
+// Sub-tiles of a launch from its tickets that hold lines, t, and the resident
+// CTAs of whole tiles (592 mixed, 296 plain).  Measured with 1 / 2 / 4
+// sub-tiles: mixed t = 40 69 / 61 / 59 us, t = 75 72 / 64 / 64, t = 150
+// 77 / 73 / 75, t = 270 81 / 83 / 99; plain t = 40 212 / 136 / 100, t = 75
+// 224 / 144 / 148, t = 150 233 / 154 / 175, t = 270 251 / 258 / 289.  The sums
+// are the same to the bit, so the choice may depend on the batch.
+static int sub_tiles(bool mixed, const VoigtPlan &pl, int64_t nlines, const GridDev &g) {
+  const int64_t tickets = pl.tiles * std::min<int64_t>(pl.nsplit, tile_chunks(g, nlines, pl.shape));
+  return 6 * tickets <= pl.ctas ? 4 : 8 * tickets <= (mixed ? 3 : 6) * (int64_t)pl.ctas ? 2 : 1;
+}
+
+VoigtPlan plan_voigt_section(bool mixed, int shape, const GridDev &g, int64_t nlines, int tile0,
+                             int ntiles, int grid_ctas, int nstates) {
   VoigtPlan pl;
   pl.shape = mixed ? shape : 0;
   pl.G = voigt_tile_points(pl.shape);
   pl.tile0 = tile0;
   pl.tiles_per_state = ntiles;
-  pl.tiles = ntiles;
+  pl.tiles = (int64_t)ntiles * nstates;
   pl.ctas = grid_ctas > 0 ? grid_ctas : voigt_ctas(mixed, pl.shape);
-  pl.nsplit = voigt_nsplit(nx, pl.shape);
+  pl.nsplit = voigt_nsplit(g, nlines, pl.shape);
   pl.partial_doubles = pl.nsplit > 1 ? (size_t)pl.tiles * pl.nsplit * pl.G : 0;
-  pl.counters = pl.nsplit > 1 ? (size_t)pl.tiles : 0;
+  pl.counters = pl.nsplit > 1 ? (size_t)pl.tiles * HK_MAX_SUB : 0;
+  pl.work_bytes = (size_t)pl.tiles * sizeof(longlong2) + pl.counters * sizeof(unsigned);
   return pl;
 }
 
-VoigtPlan plan_voigt_sum(bool mixed, int shape, int64_t nx, int nstates, int grid_ctas) {
+VoigtPlan plan_voigt_sum(bool mixed, int shape, const GridDev &g, int64_t nlines, int nstates,
+                         int grid_ctas) {
   const int G = voigt_tile_points(mixed ? shape : 0);
-  VoigtPlan pl = plan_voigt_section(mixed, shape, nx, 0, (int)((nx + G - 1) / G), grid_ctas);
-  pl.tiles = (int64_t)pl.tiles_per_state * nstates;
-  pl.partial_doubles = pl.nsplit > 1 ? (size_t)pl.tiles * pl.nsplit * pl.G : 0;
-  pl.counters = pl.nsplit > 1 ? (size_t)pl.tiles : 0;
-  return pl;
+  return plan_voigt_section(mixed, shape, g, nlines, 0, (int)((g.nx + G - 1) / G), grid_ctas, nstates);
 }
 
 cudaError_t launch_voigt_sum(bool mixed, const VoigtPlan &pl, const void *prep_d,
                              const double *nu0_d, int64_t nlines, const GridDev &g,
-                             const StateDev *states_d, unsigned *ticket_d, double *partial_d,
-                             unsigned *tile_cnt_d, double *K_d, int64_t k_stride,
-                             cudaStream_t stream) {
+                             StateDev *states_d, const unsigned long long *wbits_d,
+                             unsigned *ticket_d, double *partial_d, void *work_d, double *K_d,
+                             int64_t k_stride, cudaStream_t stream) {
   const int64_t total64 = pl.tiles * pl.nsplit;
-  if (total64 > 0x7fffffff) return cudaErrorInvalidValue;
+  if (total64 > 0x7fffffff / HK_MAX_SUB) return cudaErrorInvalidValue;
   if (pl.G != voigt_tile_points(pl.shape)) return cudaErrorInvalidValue;
   if (mixed && (g.profile >= 3 || g.plinth || g.subL) && pl.shape != 0)
     return cudaErrorInvalidValue;  // shape 0 only
-  const int total = (int)total64;
-  cudaError_t e = cudaMemsetAsync(ticket_d, 0, sizeof(unsigned), stream);
-  if (e != cudaSuccess) return e;
+  const bool g34 = mixed && g.profile >= 3;
+  const int ext = mixed ? ext_kind(g) : HK_EXT_NONE;
+  const int sub = (pl.shape == 0 && !g34 && ext == HK_EXT_NONE) ? sub_tiles(mixed, pl, nlines, g) : 1;
+  const int total = (int)total64 * sub;
   if (total <= 0) return cudaSuccess;
-  if (pl.nsplit > 1) {
-    if (!partial_d || !tile_cnt_d) return cudaErrorInvalidValue;
-    e = cudaMemsetAsync(tile_cnt_d, 0, sizeof(unsigned) * pl.counters, stream);
-    if (e != cudaSuccess) return e;
-  }
+  if (!work_d || (pl.nsplit > 1 && !partial_d)) return cudaErrorInvalidValue;
+  longlong2 *ranges = static_cast<longlong2 *>(work_d);
+  unsigned *tile_cnt_d = reinterpret_cast<unsigned *>(ranges + pl.tiles);
+  tile_range_kernel<<<(unsigned)((2 * pl.tiles + 7) / 8), 256, 0, stream>>>(
+      nu0_d, nlines, g, states_d, wbits_d, pl.G, pl.tile0, pl.tiles_per_state, pl.tiles,
+      reinterpret_cast<int64_t *>(ranges), ticket_d, tile_cnt_d, (int64_t)pl.counters);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
   const int ctas = (int)std::min<int64_t>(pl.ctas, total);
   e = with_kernel(mixed, pl.shape, [&](auto kfn, size_t smem, int threads) {
     if (smem > 48 * 1024) {
       const cudaError_t ea = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (ea != cudaSuccess) return ea;
     }
-    kfn<<<ctas, threads, smem, stream>>>(prep_d, nu0_d, nlines, g, states_d, pl.tile0,
+    kfn<<<ctas, threads, smem, stream>>>(prep_d, ranges, nlines, g, states_d, pl.tile0,
                                             pl.tiles_per_state, pl.nsplit, total, ticket_d,
                                             partial_d, tile_cnt_d, K_d, k_stride);
     return cudaGetLastError();
-  }, mixed && g.profile >= 3, mixed ? ext_kind(g) : HK_EXT_NONE);
+  }, g34, ext, sub);
   return e;
 }
 
@@ -1867,7 +1975,8 @@ static cudaError_t with_table_kernel(bool mixed, int shape, F &&f, bool g34 = fa
   }
 }
 
-TablePlan plan_table(bool mixed, int shape, int64_t nlines, int64_t nx, int nstates) {
+TablePlan plan_table(bool mixed, int shape, int64_t nlines, const GridDev &g, int nstates) {
+  const int64_t nx = g.nx;
   TablePlan tp;
   tp.shape = mixed ? shape : 0;
   tp.G = voigt_tile_points(tp.shape);
@@ -1879,7 +1988,7 @@ TablePlan plan_table(bool mixed, int shape, int64_t nlines, int64_t nx, int nsta
   tp.lpt = 4096;
   tp.npb = (int)std::max<int64_t>(1, (nlines + tp.lpt - 1) / tp.lpt);
   tp.tps = (int)((nx + tp.G - 1) / tp.G);
-  tp.nsplit = voigt_nsplit(nx, tp.shape);
+  tp.nsplit = voigt_nsplit(g, nlines, tp.shape);
   tp.nsum = (long long)tp.tps * tp.nsplit;
   tp.total = (long long)nstates * (tp.npb + tp.nsum);
   tp.ring_bytes = (size_t)tp.slots * (size_t)std::max<int64_t>(nlines, 1) * (mixed ? sizeof(LinePrepF) : sizeof(LinePrep));
