@@ -10,10 +10,10 @@
 //   optional expfx + rescale(-1) reconstruction          resample.h:497-524
 // The Householder factorisation of the Chebyshev Vandermonde matrix is done
 // once per (Nxb, nC) by qr_kernel (resample.h:14-37, 73-227), a single CTA.
-// Bins larger than the shared-memory budget run the same code on a global
-// scratch slice.
+// Bins above KD_MAX_NXB points run kdist_big_kernel on a global scratch slice.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cub/block/block_merge_sort.cuh>
 
@@ -77,8 +77,17 @@ __device__ __forceinline__ double block_sum1(double v, double *red2, int parity)
 // Vandermonde_kernel + QR_kernel (resample.h:14-37, 73-227), one CTA.
 // V is column-major nxb x nc; on return it holds the Householder vectors
 // below/on the diagonal and R above it; C, D as in the reference.
+//
+// moments = 1 (kdist_moments): the fit takes Q^T b from the bin's Chebyshev
+// moments (fit_moments) and needs, of the reflections, only the row f = e_(nc-1)^T
+// H_(nc-2) .. H_0 that gives the last element after nc - 1 of them, and the
+// matrix M that takes (A^T b, f . b) to the coefficients (both substitutions
+// with R).  f's first nc - 1 entries replace Cv[0 .. nc-2] and the others the
+// last column from row nc - 1 on; M replaces R and the heads of the
+// reflections, V[i + nxb j] for i, j < nc but for its last entry, 1 / D[nc-1].
+// Dynamic shared memory: 2 nc^2 doubles with moments, else none.
 __global__ void __launch_bounds__(KD_THREADS)
-qr_kernel(int nxb, int nc, double *__restrict__ V, double *__restrict__ Cv,
+qr_kernel(int nxb, int nc, int moments, double *__restrict__ V, double *__restrict__ Cv,
           double *__restrict__ D) {
   __shared__ double red[32];
   for (int id = threadIdx.x; id < nxb; id += blockDim.x) {
@@ -126,7 +135,68 @@ qr_kernel(int nxb, int nc, double *__restrict__ V, double *__restrict__ Cv,
       __syncthreads();
     }
   }
+  if (!moments) return;
+  // f = H_0 (H_1 ( .. H_(nc-2) e_(nc-1))), rows >= nc - 1 in the last column,
+  // the first rows in s_head
+  __shared__ double s_head[KD_MAX_NC];
+  double *f = V + (int64_t)nxb * (nc - 1);
+  for (int k = threadIdx.x; k < nxb; k += blockDim.x) {
+    if (k < nc - 1) s_head[k] = 0.0;
+    else f[k] = k == nc - 1 ? 1.0 : 0.0;
+  }
+  __syncthreads();
+  for (int j = nc - 2; j >= 0; --j) {
+    const double *vj = V + (int64_t)nxb * j;
+    double dot = 0.0;
+    for (int k = j + threadIdx.x; k < nxb; k += blockDim.x)
+      dot = __fma_rn(vj[k], k < nc - 1 ? s_head[k] : f[k], dot);
+    dot = block_sum(dot, red);
+    const double t = dot / Cv[j];
+    __syncthreads();
+    for (int k = j + threadIdx.x; k < nxb; k += blockDim.x) {
+      double &w = k < nc - 1 ? s_head[k] : f[k];
+      w = __fma_rn(-t, vj[k], w);
+    }
+    __syncthreads();
+  }
+  // column j of M: the unit vector j through the substitutions, thread j
+  extern __shared__ double qr_dyn[];
+  double *R = qr_dyn, *X = qr_dyn + nc * nc;  // X[i nc + j]: element i of column j
+  for (int q = threadIdx.x; q < nc * nc; q += blockDim.x) {
+    const int i = q / nc, j = q - i * nc;
+    R[q] = j > i ? V[i + (int64_t)nxb * j] : (i == j ? D[i] : 0.0);
+  }
+  for (int k = threadIdx.x; k < nc - 1; k += blockDim.x) Cv[k] = s_head[k];
+  __syncthreads();
+  if (threadIdx.x < nc) {
+    const int j = threadIdx.x;
+    // R^T z = e_j on the first nc - 1 rows; the last element is f . b itself
+    for (int i = 0; i < nc; ++i) {
+      double t = i == j ? 1.0 : 0.0;
+      if (i < nc - 1) {
+        for (int k = 0; k < i; ++k) t = __fma_rn(-R[k * nc + i], X[k * nc + j], t);
+        t /= R[i * nc + i];
+      }
+      X[i * nc + j] = t;
+    }
+    // R c = z (the reference's reduction keeps 64 partial sums)
+    for (int i = nc - 1; i >= 0; --i) {
+      double t = X[i * nc + j];
+      for (int k = i + 1; k < nc && k < 64; ++k) t = __fma_rn(-R[i * nc + k], X[k * nc + j], t);
+      t /= R[i * nc + i];
+      X[i * nc + j] = t;
+      if (i < nc - 1 || j < nc - 1) V[i + (int64_t)nxb * j] = t;
+    }
+  }
 }
+
+// Whether the fit of (nxb, nc) goes through the moments: the Chebyshev basis on
+// nxb equally spaced points is well conditioned for nc well below sqrt(nxb)
+// and, measured, for 6 nc <= nxb (condition number 3 - 7 from 120 points x 20
+// to 11000 x 30; coefficients within 6e-14 of the reflections').  Below 4
+// coefficients the reflections do not spread a non-finite value to all of
+// them, so those keep the reflections.
+static __host__ __device__ inline bool kdist_moments(int nxb, int nc) { return nc >= 4 && 6 * nc <= nxb; }
 
 struct KdistArgs {
   const double *K;       // nstates x nx, unsorted
@@ -138,228 +208,514 @@ struct KdistArgs {
   int *nxmin;            // nstates x nbins
   double *sorted;        // optional nstates x nx
   double *recon;         // optional nstates x nx
-  double *scratch;       // global work when the bin does not fit in smem
-  int use_smem;
+  double *scratch;       // kdist_big_kernel's work
 };
 
-struct KeyLess {
-  __device__ __forceinline__ bool operator()(uint64_t x, uint64_t y) const { return x < y; }
-};
+constexpr uint64_t KD_KEY_END = 0xffffffffffffffffull;  // after every key of a value
 
-// IPT > 0: the bin is sorted in registers, IPT keys per thread, by a block
-// merge sort (CUB's BlockMergeSort: per-thread sort, then log2(1024) rounds of
-// merge-path merges through shared memory) -- O(n log n) comparisons where
-// the bitonic network needs O(n log^2 n); its tile (1024 IPT + 1 keys) uses
-// the key array.  IPT = 0: bitonic network, one shared-memory or global pass
-// per stage (bins the merge sort does not hold).  The sorted keys are the
-// same either way: the total order of the FP64 bit patterns has no ties
-// between distinct values.
-template <int IPT>
-__global__ void __launch_bounds__(KD_THREADS)
-kdist_kernel(KdistArgs a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double red[64];
-  __shared__ int s_trans;
-  __shared__ double s_c[KD_MAX_NC], s_cv[KD_MAX_NC], s_d[KD_MAX_NC];
-  const int b = blockIdx.x, s = blockIdx.y;
-  const int nxb = a.nxb, P2 = a.pow2;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  uint64_t *keys;
-  double *work;
-  if (a.use_smem) {
-    keys = reinterpret_cast<uint64_t *>(smem_raw);
-    work = reinterpret_cast<double *>(smem_raw + (size_t)P2 * 8);
-  } else {
-    const size_t slot = ((size_t)s * a.nbins + b) * (size_t)(P2 + nxb);
-    keys = reinterpret_cast<uint64_t *>(a.scratch + slot);
-    work = a.scratch + slot + P2;
-  }
-  const double *src = a.K + (int64_t)s * a.k_stride + (int64_t)b * nxb;
-  constexpr uint64_t KEY_END = 0xffffffffffffffffull;  // after every key of a value
-  if (IPT > 0) {
-    // coalesced into shared memory, then blocked into registers
-    for (int i = tid; i < nxb; i += nt) keys[i] = f2key(src[i]);
-  } else {
-    for (int i = tid; i < P2; i += nt) keys[i] = (i < nxb) ? f2key(src[i]) : KEY_END;
-  }
-  for (int i = tid; i < a.nc; i += nt) {
-    s_cv[i] = a.Cv[i];
-    s_d[i] = a.D[i];
-  }
-  __syncthreads();
-
-  // sort, ascending
-  if (IPT > 0) {
-    constexpr int NI = IPT > 0 ? IPT : 1;
-    using Sorter = cub::BlockMergeSort<uint64_t, KD_THREADS, NI>;
-    uint64_t v[NI];
-#pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      const int k = tid * NI + i;
-      v[i] = k < nxb ? keys[k] : KEY_END;
-    }
-    __syncthreads();  // the tile storage below overlays keys[]
-    Sorter(*reinterpret_cast<typename Sorter::TempStorage *>(keys)).Sort(v, KeyLess(), nxb, KEY_END);
-#pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      const int k = tid * NI + i;
-      if (k < nxb) work[k] = key2f(v[i]);
-    }
-  } else {
-    for (int size = 2; size <= P2; size <<= 1) {
-      for (int stride = size >> 1; stride > 0; stride >>= 1) {
-        for (int i = tid; i < (P2 >> 1); i += nt) {
-          const int pos = 2 * i - (i & (stride - 1));
-          const int q = pos + stride;
-          const uint64_t x = keys[pos], y = keys[q];
-          const bool up = (pos & size) == 0;
-          if ((x > y) == up) {
-            keys[pos] = y;
-            keys[q] = x;
-          }
-        }
-        __syncthreads();
-      }
-    }
-    for (int i = tid; i < nxb; i += nt) work[i] = key2f(keys[i]);
-  }
-  __syncthreads();
-  if (a.sorted) {
-    double *dst = a.sorted + (int64_t)s * a.k_stride + (int64_t)b * nxb;
-    for (int i = tid; i < nxb; i += nt) dst[i] = work[i];
-  }
-  if (a.coeff == nullptr) return;
-
-  // findCut (resample.h:362-388) on the sorted bin.  Within a bin at most
-  // one index j has K[j] <= kmin < K[j+1]; the empty-bin rules follow it.
-  if (tid == 0) s_trans = -1;
-  __syncthreads();
-  const bool last_bin = (b == a.nbins - 1);
+// findCut (resample.h:362-388) on the sorted bin: within a bin at most one
+// index j has K[j] <= kmin < K[j+1]; the empty-bin rules follow it.  s_trans
+// holds -1 and a barrier has passed.
+__device__ __forceinline__ int find_cut(const double *work, int nxb, double kmin, bool last_bin,
+                                        int *s_trans) {
   // transitions at local j <= nxb-2; for the bin's last index the reference's
   // "complete empty bin" rule gives the same Nxb (and the state's last index
   // is never visited: id < NL-1)
-  for (int j = tid; j < nxb - 1; j += nt)
-    if (work[j] <= a.kmin && work[j + 1] > a.kmin) s_trans = j;
+  for (int j = threadIdx.x; j < nxb - 1; j += blockDim.x)
+    if (work[j] <= kmin && work[j + 1] > kmin) *s_trans = j;
   __syncthreads();
-  int nxmin = 0;
-  {
-    const int jt = s_trans;
-    if (jt >= 0) nxmin = jt + 1;
-    if (!last_bin) {
-      if (work[nxb - 1] <= a.kmin) nxmin = nxb;
-    } else if (nxb >= 3 && work[nxb - 3] <= a.kmin) {
-      // id == NL-3 rule; a transition at the later id NL-2 wins the race
-      nxmin = (jt == nxb - 2) ? nxb - 1 : nxb;
-    }
+  const int jt = *s_trans;
+  int nxmin = jt >= 0 ? jt + 1 : 0;
+  if (!last_bin) {
+    if (work[nxb - 1] <= kmin) nxmin = nxb;
+  } else if (nxb >= 3 && work[nxb - 3] <= kmin) {
+    // id == NL-3 rule; a transition at the later id NL-2 wins the race
+    nxmin = (jt == nxb - 2) ? nxb - 1 : nxb;
   }
-  if (tid == 0) a.nxmin[(int64_t)s * a.nbins + b] = nxmin;
+  return nxmin;
+}
 
-  // rescale(+1) into keys[] (reused as doubles), then copy back
-  double *tmp = reinterpret_cast<double *>(keys);
-  if (nxmin > 0) {
-    for (int j = tid; j < nxb; j += nt) {
-      double ii = __fma_rn(1.0 - nxmin / ((double)(nxb - 1)), (double)j, (double)nxmin);
-      if (ii >= nxb - 1) ii = 0.999999 * (nxb - 1);
-      const int il = (int)(ii / ((double)nxb) * nxb);
-      const double Kl = work[il], Kr = work[il + 1];
-      tmp[j] = __fma_rn(Kr - Kl, ii - il, Kl);
-    }
-    __syncthreads();
-    for (int j = tid; j < nxb; j += nt) work[j] = tmp[j];
-    __syncthreads();
-  }
-  for (int j = tid; j < nxb; j += nt) work[j] = log(work[j] * a.unitScale);
-  __syncthreads();
+// rescale(+1) of one element
+__device__ __forceinline__ double rescale_up(const double *work, int nxb, int nxmin, int j) {
+  double ii = __fma_rn(1.0 - nxmin / ((double)(nxb - 1)), (double)j, (double)nxmin);
+  if (ii >= nxb - 1) ii = 0.999999 * (nxb - 1);
+  const int il = (int)(ii / ((double)nxb) * nxb);
+  const double Kl = work[il], Kr = work[il + 1];
+  return __fma_rn(Kr - Kl, ii - il, Kl);
+}
 
-  // leastSquare_kernel: Q^T b with the first nc-1 reflections.  Thread tid
-  // owns the bin elements k = tid + n nt (k >= j) in every reflection, so a
-  // reflection needs only its block sum's barrier.
-  const int nc = a.nc;
-  if (IPT > 0) {
-    // (nxb <= 1024 IPT) the thread's entries of V's column in registers, the
-    // next column copied asynchronously into the free key array while this
-    // one is used; a thread copies and reads only its own entries
-    constexpr int NI = IPT > 0 ? IPT : 1;
-    double vv[NI];
-    double *pbuf = reinterpret_cast<double *>(keys);
-#pragma unroll
-    for (int n = 0; n < NI; ++n) {
-      const int k = tid + n * KD_THREADS;
-      vv[n] = (k < nxb && nc > 1) ? a.V[k] : 0.0;
-    }
-    for (int j = 0; j < nc - 1; ++j) {
-      const bool more = j + 1 < nc - 1;
-      if (more) {
-        const double *vnext = a.V + (int64_t)nxb * (j + 1);
-#pragma unroll
-        for (int n = 0; n < NI; ++n) {
-          const int k = tid + n * KD_THREADS;
-          if (k < nxb) {
-            const unsigned dst = (unsigned)__cvta_generic_to_shared(pbuf + k);
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(vnext + k));
-          }
-        }
-        asm volatile("cp.async.commit_group;\n" ::);
-      }
-      double dot = 0.0;
-#pragma unroll
-      for (int n = 0; n < NI; ++n) {
-        const int k = tid + n * KD_THREADS;
-        if (k < nxb && k >= j) dot = __fma_rn(vv[n], work[k], dot);
-      }
-      dot = block_sum1(dot, red, j & 1);
-      const double t = dot / s_cv[j];
-#pragma unroll
-      for (int n = 0; n < NI; ++n) {
-        const int k = tid + n * KD_THREADS;
-        if (k < nxb && k >= j) work[k] = __fma_rn(-t, vv[n], work[k]);
-      }
-      if (more) {
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-#pragma unroll
-        for (int n = 0; n < NI; ++n) {
-          const int k = tid + n * KD_THREADS;
-          vv[n] = k < nxb ? pbuf[k] : 0.0;
-        }
-      }
-    }
-  } else {
-    for (int j = 0; j < nc - 1; ++j) {
-      const double *vj = a.V + (int64_t)nxb * j;
-      double dot = 0.0;
-      for (int k = tid; k < nxb; k += nt)
-        if (k >= j) dot = __fma_rn(vj[k], work[k], dot);
-      dot = block_sum1(dot, red, j & 1);
-      const double t = dot / s_cv[j];
-      for (int k = tid; k < nxb; k += nt)
-        if (k >= j) work[k] = __fma_rn(-t, vj[k], work[k]);
-    }
+// rescale(-1) of one element of the reconstruction
+__device__ __forceinline__ double rescale_down(const double *work, int nxb, int nxmin, double kmin,
+                                               int j) {
+  if (nxmin <= 0) return work[j];
+  if (j < nxmin) return kmin;
+  double ii = (j - nxmin) / ((double)(nxb - nxmin - 1)) * (nxb - 1);
+  if (ii >= nxb - 1) ii = 0.999999 * (nxb - 1);
+  const int il = (int)(ii / ((double)nxb) * nxb);
+  const double Kl = work[il], Kr = work[il + 1];
+  return __fma_rn(Kr - Kl, ii - il, Kl);
+}
+
+// leastSquare_kernel with the reflections: Q^T b by the first nc-1 of them,
+// thread tid owning the bin elements k = tid + n nt (k >= j) in every
+// reflection (one barrier each), then the back-substitution by one thread,
+// whose result is s_c (and co).  red: 64 doubles.
+__device__ void fit_reflections(const KdistArgs &a, double *work, const double *s_cv, const double *s_d,
+                                double *red, double *s_c, double *__restrict__ co) {
+  const int nxb = a.nxb, nc = a.nc, tid = threadIdx.x, nt = blockDim.x;
+  for (int j = 0; j < nc - 1; ++j) {
+    const double *vj = a.V + (int64_t)nxb * j;
+    double dot = 0.0;
+    for (int k = tid; k < nxb; k += nt)
+      if (k >= j) dot = __fma_rn(vj[k], work[k], dot);
+    dot = block_sum1(dot, red, j & 1);
+    const double t = dot / s_cv[j];
+    for (int k = tid; k < nxb; k += nt)
+      if (k >= j) work[k] = __fma_rn(-t, vj[k], work[k]);
   }
-  // the R factor's rows used by the back-substitution, copied in parallel
-  // into the (now free) key array when it fits
-  const int lim = nc < 64 ? nc : 64;
-  double *Rb = reinterpret_cast<double *>(keys);
-  const bool rb = nc * lim <= P2;
-  if (rb)
-    for (int q = tid; q < nc * lim; q += nt) Rb[q] = a.V[q / lim + (int64_t)nxb * (q % lim)];
   __syncthreads();
   if (tid == 0) {
-    // back-substitution; the reference's reduction keeps 64 partial sums
+    // the reference's reduction keeps 64 partial sums
+    const int lim = nc < 64 ? nc : 64;
     double *bb = work;
     bb[nc - 1] /= s_d[nc - 1];
     for (int i = nc - 2; i >= 0; --i) {
       double sum = 0.0;
-      for (int j = i + 1; j < lim; ++j)
-        sum = __fma_rn(rb ? Rb[i * lim + j] : a.V[i + (int64_t)nxb * j], bb[j], sum);
+      for (int j = i + 1; j < lim; ++j) sum = __fma_rn(a.V[i + (int64_t)nxb * j], bb[j], sum);
       bb[i] = (bb[i] - sum) / s_d[i];
     }
-    double *co = a.coeff + ((int64_t)s * a.nbins + b) * nc;
     for (int i = 0; i < nc; ++i) {
       co[i] = bb[i];
       s_c[i] = bb[i];
     }
   }
   __syncthreads();
+}
+
+// The fit from the bin's Chebyshev moments m_j = sum_k T_j(x_k) b_k, j < nc-1:
+// A^T b = R^T Q^T b, so a forward substitution with R gives the first nc - 1
+// elements of Q^T b, and the last one, which the reference leaves with nc - 1
+// reflections, is f . b; the coefficients are M (m, f . b) (qr_kernel).  The
+// T_j come from their recurrence in registers, at x_k and -x_k together
+// (T_j(-x) = (-1)^j T_j(x)): 10 DFMA per point for ten moments, where the
+// reflections read 19 columns of V from L2 (1.5 MB per 10000-point bin) and
+// closed each with a block-wide sum.  The moments go in groups of KD_MG, each
+// running the recurrence up to its first.
+// buf: (groups * KD_MG + 1) * warps doubles, then M if it fits.
+constexpr int KD_MG = 10;
+template <int THREADS, int IPT>
+__device__ __forceinline__ void fit_moments(const KdistArgs &a, const double *b, const double *s_d,
+                                            double *buf, int buf_doubles, double *s_z,
+                                            double *s_c, double *__restrict__ co) {
+  constexpr int WARPS = THREADS / 32;
+  const int n = a.nxb, nc = a.nc, nm = nc - 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int groups = (nm + KD_MG - 1) / KD_MG;
+  double *Ms = buf + (groups * KD_MG + 1) * WARPS;
+  const bool in_smem = (groups * KD_MG + 1) * WARPS + nc * nc <= buf_doubles;
+  // M and f come from L2: their loads are issued before the moments' arithmetic
+  double f[IPT];
+  const double *ft = a.V + (int64_t)n * nm;  // f, rows >= nc - 1
+#pragma unroll
+  for (int i = 0; i < IPT; ++i) {
+    const int k = tid + i * THREADS;
+    f[i] = k < n ? (k < nm ? a.Cv[k] : ft[k]) : 0.0;
+  }
+  if (in_smem)
+    for (int q = tid; q < nc * nc; q += THREADS) {
+      const int j = q / nc, i = q - j * nc;
+      Ms[q] = q == nc * nc - 1 ? 1.0 / s_d[nm] : a.V[i + (int64_t)n * j];
+    }
+  double af = 0.0;
+#pragma unroll
+  for (int i = 0; i < IPT; ++i) {
+    const int k = tid + i * THREADS;
+    if (k < n) af = __fma_rn(f[i], b[k], af);
+  }
+  // (f is finite, but 0 x inf where b is not: the finite check below covers it)
+  for (int k = tid + IPT * THREADS; k < n; k += THREADS) af = __fma_rn(ft[k], b[k], af);
+  for (int o = 16; o > 0; o >>= 1) af += __shfl_xor_sync(0xffffffffu, af, o);
+  if (lane == 0) buf[groups * KD_MG * WARPS + warp] = af;
+  const double h = 2.0 / ((double)n - 1.0);
+  for (int gq = 0; gq < groups; ++gq) {
+    double acc[KD_MG];
+#pragma unroll
+    for (int q = 0; q < KD_MG; ++q) acc[q] = 0.0;
+    for (int k = tid; k < (n + 1) / 2; k += THREADS) {
+      const int k2 = n - 1 - k;
+      // (the middle point of an odd count has x = 0 to a rounding: odd T vanish)
+      const double bl = b[k], bh = k2 > k ? b[k2] : 0.0;
+      const double x = __fma_rn((double)k, h, -1.0), x2 = 2.0 * x, s = bl + bh, d = bl - bh;
+      double ta = 1.0, tb = x;
+      for (int i = 0; i < gq * KD_MG; i += 2) {
+        ta = __fma_rn(x2, tb, -ta);
+        tb = __fma_rn(x2, ta, -tb);
+      }
+#pragma unroll
+      for (int q = 0; q < KD_MG; q += 2) {
+        acc[q] = __fma_rn(ta, s, acc[q]);
+        acc[q + 1] = __fma_rn(tb, d, acc[q + 1]);
+        ta = __fma_rn(x2, tb, -ta);
+        tb = __fma_rn(x2, ta, -tb);
+      }
+    }
+    // warp sums: the first level halves the values each lane carries
+    const bool up = lane & 16;
+#pragma unroll
+    for (int q = 0; q < KD_MG / 2; ++q) {
+      const double give = up ? acc[q] : acc[q + KD_MG / 2], keep = up ? acc[q + KD_MG / 2] : acc[q];
+      acc[q] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < KD_MG / 2; ++q) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+    if ((lane & 15) == 0)
+#pragma unroll
+      for (int q = 0; q < KD_MG / 2; ++q) buf[(gq * KD_MG + q + (up ? KD_MG / 2 : 0)) * WARPS + warp] = acc[q];
+  }
+  __syncthreads();
+  // sums over the warps: value v to s_z[v], f . b to s_z[nc - 1]
+  for (int v = warp; v < nc; v += WARPS) {
+    const int src = v < nm ? v : groups * KD_MG;
+    double t = lane < WARPS ? buf[src * WARPS + lane] : 0.0;
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) s_z[v] = t;
+  }
+  __syncthreads();
+  if (tid < nc) {
+    double c = 0.0;
+    if (in_smem) {
+#pragma unroll 5
+      for (int j = 0; j < nc; ++j) c = __fma_rn(Ms[j * nc + tid], s_z[j], c);
+    } else {
+      for (int j = 0; j < nc; ++j)
+        c = __fma_rn(j == nm && tid == nm ? 1.0 / s_d[nm] : a.V[tid + (int64_t)n * j], s_z[j], c);
+    }
+    // a non-finite b (its sum is m_0) leaves no coefficient finite
+    if (!isfinite(s_z[0])) c = __longlong_as_double(0x7ff8000000000000ll);
+    co[tid] = c;
+    s_c[tid] = c;
+  }
+  __syncthreads();
+}
+
+// ------------------------------------------------- sort in shared memory
+// the low 32 bits of (v - mn) >> sh
+__device__ __forceinline__ unsigned prefix32(uint64_t v, uint64_t mn, int sh) {
+  const uint64_t u = v - mn;
+  const unsigned lo = (unsigned)u, hi = (unsigned)(u >> 32);
+  return sh < 32 ? __funnelshift_r(lo, hi, sh) : hi >> (sh - 32);
+}
+
+// Sort by distribution of the keys v of the CTA (key e = warp 32 IPT + i 32 +
+// lane in v[i], e < n), nfloor of which equal the smallest, floor, and the others
+// lie at or above mn: they go to keys[nfloor ..] in the order of their
+// prefixes (v - mn) >> sh, below KD_STEPS THREADS, each at its prefix's start
+// plus the counter's atomic, and then each finds its place among those of its
+// prefix by comparing with all of them.  False, with keys[] untouched, if more than
+// KD_RUN keys share a prefix.
+constexpr int KD_STEPS = 8, KD_RUN = 64;
+template <int THREADS, int IPT>
+__device__ __forceinline__ bool prefix_sort(const uint64_t (&v)[IPT], int n, uint64_t floor,
+                                            int nfloor, uint64_t mn, int sh, uint64_t *keys,
+                                            unsigned *cnt, int *s_scan, int *s_long) {
+  constexpr int WARPS = THREADS / 32;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint4 *c4 = reinterpret_cast<uint4 *>(cnt);
+#pragma unroll
+  for (int q = 0; q < KD_STEPS / 4; ++q) c4[tid + q * THREADS] = make_uint4(0, 0, 0, 0);
+  if (tid == 0) *s_long = 0;
+  __syncthreads();
+  const int e0 = warp * 32 * IPT + lane;
+  auto in = [&](int i) { return e0 + 32 * i < n && !(nfloor > 0 && v[i] == floor); };
+  unsigned at_[IPT];
+#pragma unroll
+  for (int i = 0; i < IPT; ++i) at_[i] = in(i) ? atomicAdd(cnt + prefix32(v[i], mn, sh), 1u) : 0u;
+  __syncthreads();
+  uint4 c[KD_STEPS / 4];
+  unsigned sum = 0, most = 0;
+#pragma unroll
+  for (int q = 0; q < KD_STEPS / 4; ++q) {
+    c[q] = c4[(KD_STEPS / 4) * tid + q];
+    sum += c[q].x + c[q].y + c[q].z + c[q].w;
+    most = max(max(most, max(c[q].x, c[q].y)), max(c[q].z, c[q].w));
+  }
+  if (most > KD_RUN) *s_long = 1;
+  unsigned incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  if (lane == 31) s_scan[warp] = (int)incl;
+  __syncthreads();
+  if (*s_long) return false;
+  unsigned at = nfloor + incl - sum;
+#pragma unroll
+  for (int w = 0; w < WARPS; ++w)
+    if (w < warp) at += s_scan[w];
+#pragma unroll
+  for (int q = 0; q < KD_STEPS / 4; ++q) {
+    uint4 o;
+    o.x = at;
+    o.y = o.x + c[q].x;
+    o.z = o.y + c[q].y;
+    o.w = o.z + c[q].z;
+    at = o.w + c[q].w;
+    c4[(KD_STEPS / 4) * tid + q] = o;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < IPT; ++i)
+    if (in(i)) {
+      at_[i] += cnt[prefix32(v[i], mn, sh)];
+      keys[at_[i]] = v[i];
+    }
+  for (int k = tid; k < nfloor; k += THREADS) keys[k] = floor;
+  __syncthreads();
+  if (sh == 0) return true;  // the prefix is the whole key
+#pragma unroll
+  for (int i = 0; i < IPT; ++i)
+    if (in(i)) {
+      const unsigned d = prefix32(v[i], mn, sh);
+      const unsigned j0 = cnt[d], j1 = d + 1 < KD_STEPS * THREADS ? cnt[d + 1] : (unsigned)n;
+      unsigned k = j0;
+      for (unsigned j = j0; j < j1; ++j) {
+        const uint64_t x = keys[j];
+        k += x < v[i] || (x == v[i] && j < at_[i]);
+      }
+      at_[i] = k;
+    }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < IPT; ++i)
+    if (in(i)) keys[at_[i]] = v[i];
+  __syncthreads();
+  return true;
+}
+
+struct KeyLess {
+  __device__ __forceinline__ bool operator()(uint64_t x, uint64_t y) const { return x < y; }
+};
+
+// The bin sorted into keys[] by a block merge sort in registers whose tile
+// (THREADS IPT + 1 keys) uses tile; out of line, so that the usual path keeps
+// its registers.
+template <int THREADS, int IPT>
+__device__ __noinline__ void merge_sort(const double *__restrict__ src, int n, void *tile, uint64_t *keys) {
+  using Sorter = cub::BlockMergeSort<uint64_t, THREADS, IPT>;
+  uint64_t v[IPT];
+#pragma unroll
+  for (int i = 0; i < IPT; ++i) {
+    const int e = threadIdx.x + i * THREADS;
+    v[i] = e < n ? f2key(src[e]) : KD_KEY_END;
+  }
+  Sorter(*static_cast<typename Sorter::TempStorage *>(tile)).Sort(v, KeyLess());
+  __syncthreads();  // the tile overlays keys[]
+#pragma unroll
+  for (int i = 0; i < IPT; ++i) {
+    const int k = threadIdx.x * IPT + i;
+    if (k < n) keys[k] = v[i];
+  }
+  __syncthreads();
+}
+
+// One CTA per (state, bin), THREADS IPT >= nxb points.
+//
+// Sort: the keys' span in the bin (largest - smallest, in the order of the
+// FP64 bit patterns; points that no line reaches, at kmin, apart) is cut to
+// KD_STEPS THREADS steps, about one per key, and prefix_sort orders the keys by
+// step and within each step.  A bin whose values crowd into few steps takes a
+// block merge sort in registers.
+// Measured, 480 bins of 10000 points (block merge sort and reflections ->
+// this): sort alone 168 -> 93 - 118 us (173 -> 189 for bins that fall back);
+// with the fit 404 -> 149 - 174; with sorted values and reconstruction written
+// 476 -> 189 - 212.  Bound: latency, one 1024-thread CTA per SM in phases
+// between barriers (load 8 %, sort 35 %, ln 10 %, moments 25 %, reconstruction
+// 16 % of a bin's time); its 115 MB of traffic would take 18 us.
+template <int THREADS, int IPT>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
+kdist_kernel(KdistArgs a) {
+  constexpr int WARPS = THREADS / 32;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double red[64];
+  __shared__ uint64_t s_mm[2 * WARPS];
+  __shared__ int s_trans, s_long, s_scan[WARPS];
+  __shared__ double s_c[KD_MAX_NC], s_cv[KD_MAX_NC], s_d[KD_MAX_NC], s_z[KD_MAX_NC];
+  const int b = blockIdx.x, s = blockIdx.y;
+  const int nxb = a.nxb;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned *cnt = reinterpret_cast<unsigned *>(smem_raw);  // KD_STEPS THREADS counters
+  uint64_t *keys = reinterpret_cast<uint64_t *>(smem_raw + sizeof(unsigned) * KD_STEPS * THREADS);
+  double *work = reinterpret_cast<double *>(keys);
+  const double *src = a.K + (int64_t)s * a.k_stride + (int64_t)b * nxb;
+
+  // the smallest key other than floor (kmin's) and the largest; how many are floor
+  const uint64_t floor = f2key(a.kmin);
+  uint64_t v[IPT], mn = KD_KEY_END, mx = 0;
+  int nf = 0;
+#pragma unroll
+  for (int i = 0; i < IPT; ++i) {
+    const int e = warp * 32 * IPT + i * 32 + lane;
+    v[i] = KD_KEY_END;
+    if (e < nxb) {
+      v[i] = f2key(src[e]);
+      if (v[i] == floor) ++nf;
+      else mn = v[i] < mn ? v[i] : mn;
+      mx = v[i] > mx ? v[i] : mx;
+    }
+  }
+  for (int i = tid; i < a.nc; i += THREADS) {
+    s_cv[i] = a.Cv[i];
+    s_d[i] = a.D[i];
+  }
+  if (tid == 0) s_trans = -1;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const uint64_t u = __shfl_xor_sync(0xffffffffu, mn, o), w = __shfl_xor_sync(0xffffffffu, mx, o);
+    mn = u < mn ? u : mn;
+    mx = w > mx ? w : mx;
+  }
+  nf = __reduce_add_sync(0xffffffffu, nf);
+  if (lane == 0) {
+    s_mm[warp] = mn;
+    s_mm[WARPS + warp] = mx;
+    s_scan[warp] = nf;
+  }
+  __syncthreads();
+  int nfloor = 0;
+#pragma unroll
+  for (int w = 0; w < WARPS; ++w) {
+    mn = s_mm[w] < mn ? s_mm[w] : mn;
+    mx = s_mm[WARPS + w] > mx ? s_mm[WARPS + w] : mx;
+    nfloor += s_scan[w];
+  }
+  if (nfloor == nxb) {
+    mn = mx;
+  } else if (nfloor > 0 && mn < floor) {
+    nfloor = 0;  // floor is not the smallest key: no key apart
+  }
+  const int bits = 64 - __clzll((long long)(mx - mn));
+  const int sh = max(0, bits - (31 - __clz(KD_STEPS * THREADS)));
+  if (!prefix_sort<THREADS, IPT>(v, nxb, floor, nfloor, mn, sh, keys, cnt, s_scan, &s_long))
+    merge_sort<THREADS, IPT>(src, nxb, smem_raw, keys);
+  double *dst = a.sorted ? a.sorted + (int64_t)s * a.k_stride + (int64_t)b * nxb : nullptr;
+  for (int i = tid; i < nxb; i += THREADS) {
+    const double x = key2f(keys[i]);
+    work[i] = x;
+    if (dst) dst[i] = x;
+  }
+  if (a.coeff == nullptr) return;
+  __syncthreads();
+  const int nxmin = find_cut(work, nxb, a.kmin, b == a.nbins - 1, &s_trans);
+  if (tid == 0) a.nxmin[(int64_t)s * a.nbins + b] = nxmin;
+  if (nxmin > 0) {
+    double t[IPT];
+#pragma unroll
+    for (int i = 0; i < IPT; ++i) {
+      const int j = tid + i * THREADS;
+      if (j < nxb) t[i] = rescale_up(work, nxb, nxmin, j);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < IPT; ++i) {
+      const int j = tid + i * THREADS;
+      if (j < nxb) work[j] = t[i];
+    }
+  }
+  __syncthreads();
+  for (int j = tid; j < nxb; j += THREADS) work[j] = log(work[j] * a.unitScale);
+  __syncthreads();
+  const int nc = a.nc;
+  double *co = a.coeff + ((int64_t)s * a.nbins + b) * nc;
+  if (kdist_moments(nxb, nc))
+    fit_moments<THREADS, IPT>(a, work, s_d, reinterpret_cast<double *>(cnt), KD_STEPS * THREADS / 2, s_z, s_c, co);
+  else
+    fit_reflections(a, work, s_cv, s_d, red, s_c, co);
+  if (a.recon == nullptr) return;
+
+  // expfx_kernel (x = -1 + 2 j / Nxb) then rescale(-1): the even and odd parts
+  // of the series at x give the values at x and -x = x_(Nxb - j)
+  const double h = 2.0 / (double)nxb, iu = 1.0 / a.unitScale;
+  for (int j = tid; j <= nxb / 2; j += THREADS) {
+    const double x = __fma_rn((double)j, h, -1.0), x2 = 2.0 * x;
+    double ta = 1.0, tb = x, ev = 0.0, od = 0.0;
+    int i = 0;
+    for (; i + 1 < nc; i += 2) {
+      ev = __fma_rn(ta, s_c[i], ev);
+      od = __fma_rn(tb, s_c[i + 1], od);
+      ta = __fma_rn(x2, tb, -ta);
+      tb = __fma_rn(x2, ta, -tb);
+    }
+    if (i < nc) ev = __fma_rn(ta, s_c[i], ev);
+    work[j] = exp(ev + od) * iu;
+    if (j > 0 && nxb - j > j) work[nxb - j] = exp(ev - od) * iu;
+  }
+  __syncthreads();
+  double *rec = a.recon + (int64_t)s * a.k_stride + (int64_t)b * nxb;
+  for (int j = tid; j < nxb; j += THREADS) rec[j] = rescale_down(work, nxb, nxmin, a.kmin, j);
+}
+
+// Bins above KD_MAX_NXB points: the same chain on a global scratch slice of
+// next_pow2(nxb) + nxb words per bin, sorted by a bitonic network.
+__global__ void __launch_bounds__(KD_THREADS)
+kdist_big_kernel(KdistArgs a) {
+  __shared__ double red[64];
+  __shared__ int s_trans;
+  __shared__ double s_c[KD_MAX_NC], s_cv[KD_MAX_NC], s_d[KD_MAX_NC], s_z[KD_MAX_NC];
+  constexpr int BUF = 4096;  // (groups KD_MG + 1) 32 at nc = 100, and M up to nc = 29
+  __shared__ double s_buf[BUF];
+  const int b = blockIdx.x, s = blockIdx.y;
+  const int nxb = a.nxb, P2 = a.pow2;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const size_t slot = ((size_t)s * a.nbins + b) * (size_t)(P2 + nxb);
+  uint64_t *keys = reinterpret_cast<uint64_t *>(a.scratch + slot);
+  double *work = a.scratch + slot + P2;
+  const double *src = a.K + (int64_t)s * a.k_stride + (int64_t)b * nxb;
+  for (int i = tid; i < P2; i += nt) keys[i] = (i < nxb) ? f2key(src[i]) : KD_KEY_END;
+  for (int i = tid; i < a.nc; i += nt) {
+    s_cv[i] = a.Cv[i];
+    s_d[i] = a.D[i];
+  }
+  if (tid == 0) s_trans = -1;
+  __syncthreads();
+  for (int size = 2; size <= P2; size <<= 1) {
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      for (int i = tid; i < (P2 >> 1); i += nt) {
+        const int pos = 2 * i - (i & (stride - 1));
+        const int q = pos + stride;
+        const uint64_t x = keys[pos], y = keys[q];
+        const bool up = (pos & size) == 0;
+        if ((x > y) == up) {
+          keys[pos] = y;
+          keys[q] = x;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  for (int i = tid; i < nxb; i += nt) work[i] = key2f(keys[i]);
+  __syncthreads();
+  if (a.sorted) {
+    double *dst = a.sorted + (int64_t)s * a.k_stride + (int64_t)b * nxb;
+    for (int i = tid; i < nxb; i += nt) dst[i] = work[i];
+  }
+  if (a.coeff == nullptr) return;
+  const int nxmin = find_cut(work, nxb, a.kmin, b == a.nbins - 1, &s_trans);
+  if (tid == 0) a.nxmin[(int64_t)s * a.nbins + b] = nxmin;
+  if (nxmin > 0) {
+    double *tmp = reinterpret_cast<double *>(keys);
+    for (int j = tid; j < nxb; j += nt) tmp[j] = rescale_up(work, nxb, nxmin, j);
+    __syncthreads();
+    for (int j = tid; j < nxb; j += nt) work[j] = tmp[j];
+  }
+  __syncthreads();
+  for (int j = tid; j < nxb; j += nt) work[j] = log(work[j] * a.unitScale);
+  __syncthreads();
+  const int nc = a.nc;
+  double *co = a.coeff + ((int64_t)s * a.nbins + b) * nc;
+  if (kdist_moments(nxb, nc)) fit_moments<KD_THREADS, 8>(a, work, s_d, s_buf, BUF, s_z, s_c, co);
+  else fit_reflections(a, work, s_cv, s_d, red, s_c, co);
   if (a.recon == nullptr) return;
 
   // expfx_kernel (x = -1 + 2 j / Nxb) then rescale(-1)
@@ -376,20 +732,7 @@ kdist_kernel(KdistArgs a) {
   }
   __syncthreads();
   double *dst = a.recon + (int64_t)s * a.k_stride + (int64_t)b * nxb;
-  for (int j = tid; j < nxb; j += nt) {
-    double Ki = work[j];
-    if (nxmin > 0) {
-      Ki = a.kmin;
-      if (j >= nxmin) {
-        double ii = (j - nxmin) / ((double)(nxb - nxmin - 1)) * (nxb - 1);
-        if (ii >= nxb - 1) ii = 0.999999 * (nxb - 1);
-        const int il = (int)(ii / ((double)nxb) * nxb);
-        const double Kl = work[il], Kr = work[il + 1];
-        Ki = __fma_rn(Kr - Kl, ii - il, Kl);
-      }
-    }
-    dst[j] = Ki;
-  }
+  for (int j = tid; j < nxb; j += nt) dst[j] = rescale_down(work, nxb, nxmin, a.kmin, j);
 }
 
 static int next_pow2(int v) {
@@ -398,19 +741,20 @@ static int next_pow2(int v) {
   return p;
 }
 
-size_t kdist_smem_bytes(int nxb) {
-  return (size_t)(next_pow2(nxb) + nxb) * 8;
-}
-
 size_t kdist_scratch_doubles(int nxb, int nbins, int nstates) {
-  const size_t need = kdist_smem_bytes(nxb);
-  if (need <= (size_t)KD_SMEM_LIMIT) return 0;
+  if (nxb <= KD_MAX_NXB) return 0;
   return (size_t)nstates * nbins * (size_t)(next_pow2(nxb) + nxb);
 }
 
 cudaError_t launch_qr(int nxb, int nc, double *V_d, double *C_d, double *D_d,
                       cudaStream_t stream) {
-  qr_kernel<<<1, KD_THREADS, 0, stream>>>(nxb, nc, V_d, C_d, D_d);
+  const bool moments = kdist_moments(nxb, nc);
+  const size_t dyn = moments ? 2 * sizeof(double) * (size_t)nc * nc : 0;
+  if (dyn > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(qr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+    if (e != cudaSuccess) return e;
+  }
+  qr_kernel<<<1, KD_THREADS, dyn, stream>>>(nxb, nc, moments, V_d, C_d, D_d);
   return cudaGetLastError();
 }
 
@@ -438,38 +782,44 @@ cudaError_t launch_kdist(const double *K_d, int64_t k_stride, int nstates,
   a.sorted = sorted_d;
   a.recon = recon_d;
   a.scratch = scratch_d;
-  const size_t smem = kdist_smem_bytes(nxb);
-  a.use_smem = smem <= (size_t)KD_SMEM_LIMIT;
-  size_t dyn = a.use_smem ? smem : 0;
-  if (!a.use_smem && scratch_d == nullptr) return cudaErrorInvalidValue;
-  // the merge sort when its tile (1024 IPT + 1 keys) fits the key array
-  int ipt = 0;
-  if (a.use_smem) {
-    static const int kIpt[] = {2, 4, 6, 8, 10, 12};
-    for (int q : kIpt)
-      if (q * KD_THREADS >= nxb && (size_t)(q * KD_THREADS + 1) <= (size_t)a.pow2) {
-        ipt = q;
-        break;
-      }
+  const dim3 grid(nbins, nstates);
+  if (nxb > KD_MAX_NXB) {
+    if (scratch_d == nullptr) return cudaErrorInvalidValue;
+    kdist_big_kernel<<<grid, KD_THREADS, 0, stream>>>(a);
+    return cudaGetLastError();
   }
-  auto run = [&](auto kfn) -> cudaError_t {
-    if (a.use_smem) {
-      cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-      if (e != cudaSuccess) return e;
-    }
-    dim3 grid(nbins, nstates);
-    kfn<<<grid, KD_THREADS, dyn, stream>>>(a);
+  auto run = [&](auto kfn, int threads, int keys) -> cudaError_t {
+    // counters and keys; the merge sort's tile overlays them
+    const size_t dyn = std::max(sizeof(unsigned) * KD_STEPS * threads + (size_t)nxb * 8,
+                                ((size_t)threads * keys + 2) * 8);
+    cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+    if (e != cudaSuccess) return e;
+    kfn<<<grid, threads, dyn, stream>>>(a);
     return cudaGetLastError();
   };
-  switch (ipt) {
-    case 2: return run(kdist_kernel<2>);
-    case 4: return run(kdist_kernel<4>);
-    case 6: return run(kdist_kernel<6>);
-    case 8: return run(kdist_kernel<8>);
-    case 10: return run(kdist_kernel<10>);
-    case 12: return run(kdist_kernel<12>);
-    default: return run(kdist_kernel<0>);
-  }
+  // 1024 threads share an SM: the smallest CTA that holds the bin at 12 keys a
+  // thread lets the barriers of one bin hide behind another's work; with
+  // fewer bins than SMs a wider CTA finishes its bin sooner
+  const int64_t ctas = (int64_t)nbins * nstates;
+  const int thr = (nxb > 6144 || ctas <= 148) ? 1024 : (nxb > 3072 || ctas <= 296) ? 512 : 256;
+  const int ipt = (nxb + thr - 1) / thr;
+#define KD_CASE(T, I) \
+  if (thr == T && ipt <= I) return run(kdist_kernel<T, I>, T, I);
+  KD_CASE(1024, 2)
+  KD_CASE(1024, 4)
+  KD_CASE(1024, 6)
+  KD_CASE(1024, 8)
+  KD_CASE(1024, 10)
+  KD_CASE(1024, 12)
+  KD_CASE(512, 4)
+  KD_CASE(512, 8)
+  KD_CASE(512, 10)
+  KD_CASE(512, 12)
+  KD_CASE(256, 4)
+  KD_CASE(256, 8)
+  KD_CASE(256, 12)
+#undef KD_CASE
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace hkb

@@ -10,9 +10,8 @@
 
 namespace hkb {
 
-// dynamic shared memory budget of one kdist CTA (sm_100: 227 KB per block,
-// minus the kernel's static shared arrays)
-constexpr int KD_SMEM_LIMIT = 224 * 1024;
+// points of a bin that the fit sorts in shared memory (12 per thread)
+constexpr int KD_MAX_NXB = 12288;
 
 // Tile shapes of the mixed Voigt kernel: lines per staged chunk x grid points
 // per tile (warps per CTA); shape 0 is the default and the plain FP64 form's
@@ -191,7 +190,6 @@ cudaError_t launch_prep_dump(const LinesDev &L, const GridDev &g,
 cudaError_t launch_profile_eval(int64_t n, const double *x_d, const double *y_d,
                                 int mixed, double *out_d, cudaStream_t stream);
 
-size_t kdist_smem_bytes(int nxb);
 size_t kdist_scratch_doubles(int nxb, int nbins, int nstates);
 
 cudaError_t launch_qr(int nxb, int nc, double *V_d, double *C_d, double *D_d,

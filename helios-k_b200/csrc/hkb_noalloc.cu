@@ -95,7 +95,7 @@ extern "C" hk_status hk_kdist_noalloc(const double *K, int nstates, int64_t nx, 
              nxb, nC, HK_NOALLOC_DOUBLES, HK_NOALLOC_DOUBLES);
     return bad(HK_ERR_RANGE, m);
   }
-  if (kdist_smem_bytes((int)nxb) > (size_t)KD_SMEM_LIMIT)
+  if (nxb > KD_MAX_NXB)
     return bad(HK_ERR_RANGE, "bin too large for the shared-memory sort (use hk_kdist)");
   double *base = nullptr;
   const hk_status st = scratch_for_current_device(&base, errbuf, errbuf_len);
