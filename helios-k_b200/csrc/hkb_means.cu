@@ -15,8 +15,10 @@
 //   Tr_j = (sum_k exp(-K_k m_j) + end weights) / (Nxb - 1) (Nxb - Nxmin) / Nxb
 //          + exp(-kmin m_j) Nxmin / Nxb.
 // One CTA per (state, bin) stages the bin in shared memory once; each warp
-// takes values j and sums its exponentials lane-strided with a shuffle tree
-// (no block barrier per j, where the reference reduces 512 threads per j).
+// takes values j (no block barrier per j, where the reference reduces 512
+// threads per j).  Blocks of TR_B consecutive values whose spread times m_j is
+// small -- most blocks of a sorted bin, at most m_j -- are one exponential and
+// a polynomial; the others are summed value by value.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -83,10 +85,12 @@ means_partial_kernel(const double *__restrict__ K, int64_t k_stride, GridDev g,
 __global__ void means_final_kernel(const double *__restrict__ K, int64_t k_stride, GridDev g,
                                    const double *__restrict__ T, int nchunk,
                                    const double *__restrict__ part, double *__restrict__ out) {
-  const int s = blockIdx.x, q = threadIdx.x;
-  if (q >= 4) return;
+  // warp q adds the chunks of sum q: lane-strided, then a shuffle tree
+  const int s = blockIdx.x, q = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double v = 0.0;
-  for (int c = 0; c < nchunk; ++c) v += part[((int64_t)s * nchunk + c) * 4 + q];
+  for (int c = lane; c < nchunk; c += 32) v += part[((int64_t)s * nchunk + c) * 4 + q];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane != 0) return;
   const double *Ks = K + (int64_t)s * k_stride;
   const int64_t n = g.nx;
   for (int idy = 0; idy < 3 && n >= 3; ++idy) {
@@ -118,34 +122,114 @@ cudaError_t launch_means(const double *K_d, int64_t k_stride, const GridDev &g, 
   means_partial_kernel<<<grid, MN_THREADS, 0, stream>>>(K_d, k_stride, g, T_d, nchunk, scratch_d);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  means_final_kernel<<<nstates, 32, 0, stream>>>(K_d, k_stride, g, T_d, nchunk, scratch_d, out_d);
+  means_final_kernel<<<nstates, 128, 0, stream>>>(K_d, k_stride, g, T_d, nchunk, scratch_d, out_d);
   return cudaGetLastError();
 }
 
 // ------------------------------------------------------------ transmission
 constexpr int TR_THREADS = 1024;
-constexpr int TR_SMEM_MAX = 200 * 1024;  // bins above stay in global memory (L2)
+constexpr int TR_SMEM_MAX = 200 * 1024;  // values that do not fit stay in global memory (L2)
+// Sum over a block of exp(-K_k m) = exp(-c m) sum_k exp(-(K_k - c) m), c the middle
+// of the block's values and h their half spread: for d = h m <= 1 its Taylor
+// series to degree TR_P leaves d^19 / 19! < 1e-17, with the block's power
+// sums sum_k ((K_k - c) / h)^p / p! formed once per bin.
+constexpr int TR_B = 32, TR_P = 18;
 
+// doubles of shared memory per block: c, h, the smallest value, TR_P + 1 sums
+constexpr int TR_W = TR_P + 4;
+static size_t tr_words(int nxb) { return (size_t)((nxb + TR_B - 1) / TR_B) * TR_W * sizeof(double); }
+
+// 180 bins of 10000 values x 1000 m_j: 4.58 ms with an exponential per value
+// (1.8e9 of them), 0.59 ms so (about 40 of 313 blocks per m_j still value by
+// value).  Bound: instruction issue (77 % of slots; FP64 pipe 43 %).
 __global__ void __launch_bounds__(TR_THREADS)
 transmission_kernel(const double *__restrict__ K, int64_t k_stride, int nxb, int nbins,
                     const int *__restrict__ nxmin, double kmin, int nTr, double dTr, int use_smem,
-                    double *__restrict__ Tr) {
+                    int poly_ok, double *__restrict__ Tr) {
   extern __shared__ __align__(16) double kb_s[];
   const int b = blockIdx.x, s = blockIdx.y;
   const double *src = K + (int64_t)s * k_stride + (int64_t)b * nxb;
   const double *kb = src;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nblk = (nxb + TR_B - 1) / TR_B;
+  // block q's words at w[word nblk + q]
+  double *w = use_smem ? kb_s + nxb : kb_s;
   if (use_smem) {
     for (int k = threadIdx.x; k < nxb; k += TR_THREADS) kb_s[k] = src[k];
     __syncthreads();
     kb = kb_s;
   }
+  if (poly_ok) {
+    for (int q = threadIdx.x; q < nblk; q += TR_THREADS) {
+      // (each lane starts at another value of its block: no bank conflicts)
+      const int k0 = q * TR_B, nk = min(TR_B, nxb - k0);
+      double lo = kb[k0], hi = lo;
+      bool finite = true;
+      for (int i = 0; i < TR_B; ++i) {
+        const int k = (i + lane) & (TR_B - 1);
+        if (k >= nk) continue;
+        const double v = kb[k0 + k];
+        lo = fmin(lo, v);
+        hi = fmax(hi, v);
+        finite = finite && isfinite(v);
+      }
+      const double c = 0.5 * lo + 0.5 * hi, h = 0.5 * hi - 0.5 * lo, ih = h > 0.0 ? 1.0 / h : 0.0;
+      // (a spread too small to divide by, or a value that is not finite: value by value)
+      const bool ok = finite && (h == 0.0 || isfinite(ih));
+      double a[TR_P + 1];
+#pragma unroll
+      for (int p = 0; p <= TR_P; ++p) a[p] = 0.0;
+      for (int i = 0; i < TR_B; ++i) {
+        const int k = (i + lane) & (TR_B - 1);
+        if (k >= nk) continue;
+        const double t = (kb[k0 + k] - c) * ih;
+        double tp = 1.0;
+#pragma unroll
+        for (int p = 0; p <= TR_P; ++p) {
+          a[p] += tp;
+          tp *= t;
+        }
+      }
+      w[q] = c;
+      w[nblk + q] = ok ? h : CUDART_INF;
+      w[2 * nblk + q] = finite ? lo : -CUDART_INF;
+      double f = 1.0;
+#pragma unroll
+      for (int p = 0; p <= TR_P; ++p) {
+        w[(3 + p) * nblk + q] = a[p] * f;
+        f *= -1.0 / (p + 1.0);  // (-1)^p / p!
+      }
+    }
+    __syncthreads();
+  }
   const int nm = nxmin ? nxmin[(int64_t)s * nbins + b] : 0;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double *out = Tr + ((int64_t)s * nbins + b) * nTr;
-  for (int j = warp; j < nTr; j += TR_THREADS / 32) {
+  // this CTA's share of the m_j (gridDim.z of them per bin)
+  for (int j = blockIdx.z * (TR_THREADS / 32) + warp; j < nTr; j += gridDim.z * (TR_THREADS / 32)) {
     const double m = exp((double)(j - nTr / 2) * dTr);
     double a = 0.0;
-    for (int k = lane; k < nxb; k += 32) a += exp(-kb[k] * m);
+    if (poly_ok) {
+      for (int q0 = 0; q0 < nblk; q0 += 32) {
+        const int q = q0 + lane;
+        const double d = q < nblk ? w[nblk + q] * m : 0.0;
+        // (beyond 700 the factor exp(-c m) would be subnormal)
+        const bool poly = q < nblk && d <= 1.0 && w[q] * m < 700.0;
+        // exp(-x) is 0 beyond x = 745.2
+        bool each = q < nblk && !poly && !(w[2 * nblk + q] * m > 746.0);
+        if (poly) {
+          double t = w[(3 + TR_P) * nblk + q];
+#pragma unroll
+          for (int p = TR_P - 1; p >= 0; --p) t = __fma_rn(t, d, w[(3 + p) * nblk + q]);
+          a = __fma_rn(exp(-w[q] * m), t, a);
+        }
+        for (unsigned e = __ballot_sync(0xffffffffu, each); e; e &= e - 1) {
+          const int k = (q0 + __ffs(e) - 1) * TR_B + lane;
+          if (k < nxb) a += exp(-kb[k] * m);
+        }
+      }
+    } else {
+      for (int k = lane; k < nxb; k += 32) a += exp(-kb[k] * m);
+    }
     for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
     if (lane == 0) {
       for (int idy = 0; idy < 3 && nxb >= 3; ++idy) {
@@ -164,16 +248,34 @@ cudaError_t launch_transmission(const double *K_d, int64_t k_stride, int nstates
                                 int nbins, const int *nxmin_d, double kmin, int nTr, double dTr,
                                 double *Tr_d, cudaStream_t stream) {
   if (nstates <= 0 || nbins <= 0 || nTr <= 0) return cudaSuccess;
-  const size_t smem = (size_t)nxb * sizeof(double);
-  const int use_smem = smem <= (size_t)TR_SMEM_MAX;
-  if (use_smem && smem > 48 * 1024) {
+  const size_t words = tr_words(nxb), vals = (size_t)nxb * sizeof(double);
+  const int poly_ok = words <= (size_t)TR_SMEM_MAX;
+  const int use_smem = vals + (poly_ok ? words : 0) <= (size_t)TR_SMEM_MAX;
+  const size_t smem = (use_smem ? vals : 0) + (poly_ok ? words : 0);
+  if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(transmission_kernel,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  dim3 grid(nbins, nstates);
-  transmission_kernel<<<grid, TR_THREADS, use_smem ? smem : 0, stream>>>(
-      K_d, k_stride, nxb, nbins, nxmin_d, kmin, nTr, dTr, use_smem, Tr_d);
+  // One CTA per SM (registers): the m_j of a bin are shared by as many CTAs as
+  // waste the least of the last wave; staging a bin and its power sums again
+  // costs about 2 % of its 1000 sums.
+  int dev = 0, nsm = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const int64_t bins = (int64_t)nbins * nstates;
+  int share = 1;
+  double best = 0.0;
+  for (int z = 1; z <= 8 && z * TR_THREADS / 32 <= std::max(nTr, TR_THREADS / 32); ++z) {
+    const double cost = (double)((bins * z + nsm - 1) / nsm) * (1.0 / z + 0.02 * 1000.0 / nTr);
+    if (z == 1 || cost < best) {
+      best = cost;
+      share = z;
+    }
+  }
+  dim3 grid(nbins, nstates, share);
+  transmission_kernel<<<grid, TR_THREADS, smem, stream>>>(
+      K_d, k_stride, nxb, nbins, nxmin_d, kmin, nTr, dTr, use_smem, poly_ok, Tr_d);
   return cudaGetLastError();
 }
 
