@@ -159,10 +159,20 @@ constexpr size_t smem_mixed() {
                              : sizeof(double) * SH::WARPS * HK_FN * (SH::G / SUB / HK_FB));
 }
 
+// Staged line record of the plain FP64 form; C1 .. D0: region B as in RecF,
+// S1 t4 = (s (S1 s + C1) + C0) / (((s + D2) s + D1) s + D0).
 struct __align__(16) RecD {
   double nu, iad, y2, y, S1, Sc, ey, pl;  // pl: plinth (removePlinth), else 0
-  int i0, b0, c0, c1, b1, i1, p0, p1;
+  double C1, C0, D2, D1, D0, sig1;        // sig1: region C's constant (FP64)
+  int i0, b0, c0, c1, b1, i1, wide, p1;   // wide: x^2 + y^2 may pass 1e300
 };
+
+// Shared memory of one plain CTA: staged records, the per-line region-C tables
+// and the tile's region-C sums.
+template <class SH, int SUB = 1>
+constexpr size_t smem_plain() {
+  return sizeof(RecD) * SH::CH + sizeof(double) * SH::CH * HK_D916_MR + sizeof(double) * (SH::G / SUB);
+}
 
 // first index in [0, n) with a[idx] >= v (n if none); all 32 lanes call it
 __device__ int64_t lower_bound_warp(const double *__restrict__ a, int64_t n,
@@ -441,8 +451,8 @@ __device__ __forceinline__ void stage_rtab(float y, float *__restrict__ Rtab) {
 }
 
 template <bool CG>
-__device__ __forceinline__ void stage_plain(const LinePrep *__restrict__ P, int64_t l,
-                                            int64_t g0, int64_t g1, RecD *recp) {
+__device__ __forceinline__ void stage_plain(const LinePrep *__restrict__ P, const GridDev &g, int64_t l,
+                                            int64_t g0, int64_t g1, RecD *recp, double *ftab) {
   const LinePrep lp = load_record<CG>(P + l);
   int li[6] = {clip_local(lp.i0, g0, g1), clip_local(lp.b0, g0, g1),
                clip_local(lp.c0, g0, g1), clip_local(lp.c1, g0, g1),
@@ -463,7 +473,30 @@ __device__ __forceinline__ void stage_plain(const LinePrep *__restrict__ P, int6
   r.c1 = li[3];
   r.b1 = li[4];
   r.i1 = nonempty ? li[5] : 0;
-  r.p0 = r.p1 = 0;
+  r.p1 = 0;
+  const double Y = r.y2;
+  const double A2 = 2.0 * Y + (3.0 - 6.0 / CUDART_PI), B2 = (Y + 1.5) * (Y + 1.5);
+  r.C1 = lp.S1 * (2.0 * Y + (2.5 - 4.0 / CUDART_PI));
+  r.C0 = lp.S1 * ((Y + 1.5) * (Y + 1.0));
+  r.D2 = A2 + Y;
+  r.D1 = __fma_rn(A2, Y, B2);
+  r.D0 = B2 * Y;
+  const double xa = (grid_x(g, g0) - lp.nu) * lp.iad, xb = (grid_x(g, g1 - 1) - lp.nu) * lp.iad;
+  r.wide = !(fmax(xa * xa, xb * xb) + Y < 1e300);
+  r.sig1 = 0.0;
+  if (nonempty && li[3] > li[2]) {
+    // region C in the tile: the denominators and the x-independent sum
+    double e = exp(-HK_D916_A2), q = exp(-3.0 * HK_D916_A2);  // exp(-a^2 m^2) by its ratios
+    for (int m = 1; m <= HK_D916_MR; ++m) {
+      const double f = 1.0 / __fma_rn(HK_D916_A2 * m, (double)m, Y);
+      ftab[m - 1] = f;
+      if (m <= HK_D916_K) {
+        r.sig1 = __fma_rn(e, f, r.sig1);
+        e *= q;
+        q *= 0.606538354524358;  // exp(-2 a^2)
+      }
+    }
+  }
   *recp = r;
 }
 
@@ -1002,11 +1035,20 @@ __device__ __forceinline__ void sweep_pl64(const RecF &r, const ExtPL &pe, int w
 }
 
 // ------------------------------------------------------------ FP64 sweep
+// One FP64 division per pair and, in region C, four exponentials and three
+// divisions per term of the series bounded it: now a region-B pair is 13 FP64
+// operations (GH2 as one quotient of polynomials with every coefficient
+// positive, rcp_d) and region C, its points packed over the lanes, takes its
+// denominators from a table per staged line (voigt916_tab_d).  6e4 lines x 3e5
+// points: 1216 -> 625 us.  Now latency: 16 warps per SM at 128 registers (80
+// registers for 24 warps spill: 695 us), FP64 pipe 32 %.
 template <int PPL>
 __device__ __forceinline__ void sweep_plain(const RecD &r, int wb, int lane,
                                             const double (&xg)[PPL],
                                             double (&acc)[PPL], const GridDev &g,
-                                            const StateDev &st) {
+                                            const StateDev &st, int64_t g0,
+                                            const double *__restrict__ ftab,
+                                            double *__restrict__ cacc) {
   const int we = wb + 32 * PPL;
   if (r.i1 <= wb || r.i0 >= we) return;
   if (g.profile != 1 || g.plinth || g.subL) {
@@ -1030,33 +1072,47 @@ __device__ __forceinline__ void sweep_plain(const RecD &r, int wb, int lane,
     }
     return;
   }
+  const double S1 = r.S1, Y = r.y2, nu = r.nu, iad = r.iad;
   const bool full = r.i0 <= wb && r.i1 >= we;
-  if (full && ((r.b0 <= wb && r.c0 >= we) || (r.c1 <= wb && r.b1 >= we))) {
+  if (full && !r.wide && ((r.b0 <= wb && r.c0 >= we) || (r.c1 <= wb && r.b1 >= we))) {
+    const double C1 = r.C1, C0 = r.C0, D2 = r.D2, D1 = r.D1, D0 = r.D0;
 #pragma unroll
     for (int p = 0; p < PPL; ++p) {
-      const double x = (xg[p] - r.nu) * r.iad;
-      acc[p] += r.S1 * gh2_d(x, r.y2);
+      const double x = (xg[p] - nu) * iad, s = x * x;
+      acc[p] = __fma_rn(__fma_rn(s, __fma_rn(S1, s, C1), C0),
+                        rcp_d(__fma_rn(__fma_rn(s + D2, s, D1), s, D0)), acc[p]);
     }
-  } else if (full && (r.b0 >= we || r.b1 <= wb)) {
+  } else if (full && !r.wide && (r.b0 >= we || r.b1 <= wb)) {
 #pragma unroll
     for (int p = 0; p < PPL; ++p) {
-      const double x = (xg[p] - r.nu) * r.iad;
-      acc[p] += r.S1 / (x * x + r.y2);
+      const double x = (xg[p] - nu) * iad;
+      acc[p] = __fma_rn(S1, rcp_d(__fma_rn(x, x, Y)), acc[p]);
     }
   } else {
+    // (the same operations per point as above: a slice of another width, in a
+    // sub-tile, gives the same bits)
 #pragma unroll
     for (int p = 0; p < PPL; ++p) {
       const int k = wb + lane + 32 * p;
-      if (k >= r.i0 && k < r.i1) {
-        const double x = (xg[p] - r.nu) * r.iad;
-        double v;
-        if (k >= r.c0 && k < r.c1) v = r.Sc * voigt916_d(x, r.y, r.ey);
-        else if (k >= r.b0 && k < r.b1) v = r.S1 * gh2_d(x, r.y2);
-        else v = r.S1 / (x * x + r.y2);
-        acc[p] += v;
+      if (k >= r.i0 && k < r.i1 && !(k >= r.c0 && k < r.c1)) {
+        const double x = (xg[p] - nu) * iad, s = x * x;
+        if (k >= r.b0 && k < r.b1)
+          acc[p] = __fma_rn(__fma_rn(s, __fma_rn(S1, s, r.C1), r.C0),
+                            rcp_d(__fma_rn(__fma_rn(s + r.D2, s, r.D1), s, r.D0)), acc[p]);
+        else if (r.wide) acc[p] += S1 / (s + Y);
+        else acc[p] = __fma_rn(S1, rcp_d(__fma_rn(x, x, Y)), acc[p]);
       }
     }
   }
+  // region C, its points packed over the lanes, into the shared sums
+  const int lo = max(r.c0, wb), hi = min(r.c1, we);
+  if (lo >= hi) return;
+  __syncwarp();
+  for (int k = lo + lane; k < hi; k += 32) {
+    const double x = (grid_x(g, g0 + k) - nu) * iad;
+    cacc[k] = __fma_rn(r.Sc, voigt916_tab_d(x, r.y, r.ey, r.sig1, ftab), cacc[k]);
+  }
+  __syncwarp();
 }
 
 // add the FP32 sums of level lev into the FP64 sums (exact unscale) and
@@ -1120,8 +1176,10 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t
   static_assert(!FAR || (G / HK_FB <= 32 && SL % HK_FB == 0), "far-field block layout");
   Rec *rec = reinterpret_cast<Rec *>(smem_dyn);
   float *Rtab = reinterpret_cast<float *>(smem_dyn + sizeof(Rec) * CH) + HK_RPAD;
-  double *cacc = reinterpret_cast<double *>(smem_dyn + sizeof(Rec) * CH +
-                                            sizeof(float) * (HK_RPAD + CH * HK_C916_MR));
+  double *ftab = reinterpret_cast<double *>(smem_dyn + sizeof(Rec) * CH);  // plain: region C
+  double *cacc = MIXED ? reinterpret_cast<double *>(smem_dyn + sizeof(Rec) * CH +
+                                                    sizeof(float) * (HK_RPAD + CH * HK_C916_MR))
+                       : ftab + CH * HK_D916_MR;
   __shared__ int s_last;
   __shared__ int s_kcnt[CH / 32][HK_NKEY];  // staged lines per (staging warp, key)
   const int tid = threadIdx.x;
@@ -1161,10 +1219,10 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t
         kf[p >> 1].x = (float)k;
         a32[p >> 1].x = 0.f;
       }
-      cacc[k] = 0.0;  // owned by this lane only: no barrier needed
     } else {
       xg[p] = grid_x(g, g0 + k);
     }
+    cacc[k] = 0.0;  // owned by this warp only: no barrier needed
   }
 
   // Chunk c holds the lines L0 + c + q*nch (q < CH): every chunk spans
@@ -1213,7 +1271,8 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t
         if (r.c1 > r.c0 && r.i1 > r.i0) stage_rtab(r.y, Rtab + pos * HK_C916_MR);
       }
     } else if (tid < cnt_c) {
-      stage_plain<CG>(P, L0 + c + (int64_t)tid * nch, g0, g1, reinterpret_cast<RecD *>(rec) + tid);
+      stage_plain<CG>(P, g, L0 + c + (int64_t)tid * nch, g0, g1, reinterpret_cast<RecD *>(rec) + tid,
+                      ftab + tid * HK_D916_MR);
     }
     __syncthreads();
     if (MIXED) {
@@ -1376,7 +1435,8 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t
       }
     } else {
       for (int j = 0; j < cnt_c; ++j)
-        sweep_plain<PPL>(reinterpret_cast<const RecD &>(rec[j]), wb, lane, xg, acc, g, st);
+        sweep_plain<PPL>(reinterpret_cast<const RecD &>(rec[j]), wb, lane, xg, acc, g, st, g0,
+                         ftab + j * HK_D916_MR, cacc);
     }
     __syncthreads();
   }
@@ -1407,7 +1467,7 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t
     for (int p = 0; p < PPL; ++p) {
       const int k = wb + lane + 32 * p;
       const int64_t gi = g0 + k;
-      if (MIXED) acc[p] = cacc[k];
+      acc[p] = MIXED ? cacc[k] : acc[p] + cacc[k];
       if (gi < g1) Ks[gi] = st.kmin + acc[p];
     }
   } else {
@@ -1418,7 +1478,7 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t
 #pragma unroll
     for (int p = 0; p < PPL; ++p) {
       const int k = wb + lane + 32 * p;
-      if (MIXED) acc[p] = cacc[k];
+      acc[p] = MIXED ? cacc[k] : acc[p] + cacc[k];
       pt[(int64_t)part * G + k] = acc[p];
     }
     __threadfence();
@@ -1794,14 +1854,14 @@ static cudaError_t with_kernel(bool mixed, int shape, F &&f, bool g34 = false, i
     return mixed ? f((KFn)voigt_sum_kernel<true, Shape0, false, HK_EXT_NONE, n>,                      \
                      smem_mixed<Shape0, HK_EXT_NONE, n>(), Shape0::THREADS)                           \
                  : f((KFn)voigt_sum_kernel<false, Shape0, false, HK_EXT_NONE, n>,                     \
-                     sizeof(RecD) * Shape0::CH, Shape0::THREADS);
+                     smem_plain<Shape0, n>(), Shape0::THREADS);
   switch (sub) {
     HK_SUB_CASE(2)
     HK_SUB_CASE(HK_MAX_SUB)
     default: break;
   }
 #undef HK_SUB_CASE
-  if (!mixed) return f((KFn)voigt_sum_kernel<false, Shape0>, sizeof(RecD) * Shape0::CH, Shape0::THREADS);
+  if (!mixed) return f((KFn)voigt_sum_kernel<false, Shape0>, smem_plain<Shape0>(), Shape0::THREADS);
   if (g34 && ext == HK_EXT_PL)
     return f((KFn)voigt_sum_kernel<true, Shape0, true, HK_EXT_PL>, smem_mixed<Shape0, HK_EXT_PL>(),
              Shape0::THREADS);
@@ -1876,8 +1936,8 @@ int voigt_nsplit(const GridDev &g, int64_t nlines, int shape) {
 // Sub-tiles of a launch from its tickets that hold lines, t, and the resident
 // CTAs of whole tiles (592 mixed, 296 plain).  Measured with 1 / 2 / 4
 // sub-tiles: mixed t = 40 69 / 61 / 59 us, t = 75 72 / 64 / 64, t = 150
-// 77 / 73 / 75, t = 270 81 / 83 / 99; plain t = 40 212 / 136 / 100, t = 75
-// 224 / 144 / 148, t = 150 233 / 154 / 175, t = 270 251 / 258 / 289.  The sums
+// 77 / 73 / 75, t = 270 81 / 83 / 99; plain t = 40 112 / 79 / 73, t = 75
+// 119 / 85 / 114, t = 150 131 / 89 / 126, t = 270 137 / 142 / 202.  The sums
 // are the same to the bit, so the choice may depend on the batch.
 static int sub_tiles(bool mixed, const VoigtPlan &pl, int64_t nlines, const GridDev &g) {
   const int64_t tickets = pl.tiles * std::min<int64_t>(pl.nsplit, tile_chunks(g, nlines, pl.shape));
@@ -1949,7 +2009,7 @@ static cudaError_t with_table_kernel(bool mixed, int shape, F &&f, bool g34 = fa
   using KFn = void (*)(LinesDev, GridDev, const StateDev *, TableSched, void *, double *, unsigned *,
                        unsigned long long *, unsigned long long *, unsigned *, unsigned *, unsigned *,
                        TableFin *, int *, double *, int64_t);
-  if (!mixed) return f((KFn)voigt_table_kernel<false, Shape0>, sizeof(RecD) * Shape0::CH, Shape0::THREADS);
+  if (!mixed) return f((KFn)voigt_table_kernel<false, Shape0>, smem_plain<Shape0>(), Shape0::THREADS);
   if (g34 && ext == HK_EXT_PL)
     return f((KFn)voigt_table_kernel<true, Shape0, true, HK_EXT_PL>, smem_mixed<Shape0, HK_EXT_PL>(),
              Shape0::THREADS);
