@@ -118,20 +118,17 @@ __device__ __forceinline__ bool win_pred(const WinCtx &c, int kind, int64_t i,
 
 // First index in [lo, hi) where the monotone predicate holds (hi if none).
 // The answer does not depend on the estimate e (galloping + bisection).
-static __device__ __noinline__ int64_t first_true(const WinCtx &c, int kind, double R,
-                                           int64_t lo, int64_t hi, int64_t e) {
-  if (lo >= hi) return lo;
-  if (e < lo) e = lo;
-  if (e > hi) e = hi;
-  int64_t a, b;
+static __device__ __noinline__ int first_true_search(const WinCtx &c, int kind, double R, int lo,
+                                                     int hi, int e) {
+  int a, b;
   if (e >= hi || win_pred(c, kind, e, R)) {
     b = e;
     int64_t step = 1;
     while (true) {
       const int64_t t = b - step;
       if (t < lo) { a = lo; break; }
-      if (!win_pred(c, kind, t, R)) { a = t + 1; break; }
-      b = t;
+      if (!win_pred(c, kind, t, R)) { a = (int)t + 1; break; }
+      b = (int)t;
       step *= 2;
     }
   } else {
@@ -140,38 +137,50 @@ static __device__ __noinline__ int64_t first_true(const WinCtx &c, int kind, dou
     while (true) {
       const int64_t t = a - 1 + step;
       if (t >= hi) { b = hi; break; }
-      if (win_pred(c, kind, t, R)) { b = t; break; }
-      a = t + 1;
+      if (win_pred(c, kind, t, R)) { b = (int)t; break; }
+      a = (int)t + 1;
       step *= 2;
     }
   }
   while (a < b) {
-    const int64_t m = a + (b - a) / 2;
+    const int m = a + (b - a) / 2;
     if (win_pred(c, kind, m, R)) b = m;
     else a = m + 1;
   }
   return a;
 }
 
+// The same with the estimate tried first: almost every estimate of
+// line_windows is the answer, and two predicates say so; the search (out of
+// line) takes the others.
+template <int KIND>
+__device__ __forceinline__ int first_true(const WinCtx &c, double R, int lo, int hi, int e) {
+  if (lo >= hi) return lo;
+  e = min(max(e, lo), hi);
+  const bool at = e >= hi || win_pred(c, KIND, e, R);
+  const bool before = e > lo && win_pred(c, KIND, e - 1, R);
+  if (at && !before) return e;
+  return first_true_search(c, KIND, R, lo, hi, e);
+}
+
 // A starting index for first_true (any value gives the same answer; a
 // close one saves steps): idnu = 1 / dnu.
-__device__ __forceinline__ int64_t est_index(double edge, const GridDev &g,
-                                             int64_t hi, double idnu) {
+__device__ __forceinline__ int est_index(double edge, const GridDev &g, int hi, double idnu) {
   const double e = ceil((edge - g.numin) * idnu);
   if (!(e > -1.0)) return 0;
   if (e > (double)hi) return hi;
-  return (int64_t)e;
+  return (int)e;
 }
 
 // Profiles 2-4 have no regions B and C: the whole cut window is region A
 // (nuLimits_kernel voigt.h:2250, "profile != 1"; only Line6A runs for them).
 // Window boundaries of one line restricted to grid indices [g0, g1):
 // out[0..5] = i0, b0, c0, c1, b1, i1 (absolute indices, each clipped to
-// [g0, g1]).  Equals clip(oracle window) because every predicate is
+// [g0, g1]; a grid has fewer than 2^31 points).  Equals clip(oracle window) because every predicate is
 // monotone on the range it is searched over.
 __device__ __forceinline__ void line_windows(const GridDev &g, const StateDev &st,
-                                             const LineState &ls, int64_t g0,
-                                             int64_t g1, int64_t out[6]) {
+                                             const LineState &ls, int g0, int g1,
+                                             int out[6]) {
   if (ls.S == 0.0 || !(ls.iad > 0.0)) {
     for (int k = 0; k < 6; ++k) out[k] = g0;
     return;
@@ -190,23 +199,23 @@ __device__ __forceinline__ void line_windows(const GridDev &g, const StateDev &s
   // the searches' starting points need no exact arithmetic (FP64 division
   // and square root are slow on this part)
   const double idnu = 1.0 / g.dnu;
-  const int64_t i0 = first_true(c, HK_P_LEFT_CUT, 0.0, g0, g1, est_index(ls.nu - w, g, g1, idnu));
-  const int64_t i1 = first_true(c, HK_P_RIGHT_CUT, 0.0, i0, g1, est_index(ls.nu + w, g, g1, idnu));
+  const int i0 = first_true<HK_P_LEFT_CUT>(c, 0.0, g0, g1, est_index(ls.nu - w, g, g1, idnu));
+  const int i1 = first_true<HK_P_RIGHT_CUT>(c, 0.0, i0, g1, est_index(ls.nu + w, g, g1, idnu));
   if (i1 <= i0) {
     for (int k = 0; k < 6; ++k) out[k] = i0;
     return;
   }
-  const int64_t ic = first_true(c, HK_P_CENTER, 0.0, i0, i1, est_index(ls.nu, g, g1, idnu));
+  const int ic = first_true<HK_P_CENTER>(c, 0.0, i0, i1, est_index(ls.nu, g, g1, idnu));
   const double Rs[2] = {1.0e6, 100.0};
-  int64_t lohi[2][2];
+  int lohi[2][2];
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const double R = Rs[r];
     const double h2 = R - c.vy2;
     if (g.profile == 1 && h2 > 0.0) {  // regions B and C are the Voigt profile's
       const double h = (double)(sqrtf((float)h2) / (float)c.iad);
-      lohi[r][0] = first_true(c, HK_P_LEFT_R, R, i0, ic, est_index(ls.nu - h, g, g1, idnu));
-      lohi[r][1] = first_true(c, HK_P_RIGHT_R, R, ic, i1, est_index(ls.nu + h, g, g1, idnu));
+      lohi[r][0] = first_true<HK_P_LEFT_R>(c, R, i0, ic, est_index(ls.nu - h, g, g1, idnu));
+      lohi[r][1] = first_true<HK_P_RIGHT_R>(c, R, ic, i1, est_index(ls.nu + h, g, g1, idnu));
     } else {
       lohi[r][0] = ic;
       lohi[r][1] = ic;
@@ -437,9 +446,8 @@ __device__ __forceinline__ double c916_e(int m) {
   return exp(-(a * a * m * m));
 }
 // e[m-1] = c916_e(m) (a line-independent table, e.g. in shared memory).
-// Each term takes the correctly rounded reciprocal of its denominator
-// (__drcp_rn, a few instructions) times e_m instead of an FP64 division;
-// the sum is rounded to FP32 for the region-C evaluator.
+// Each term takes rcp_d of its denominator times e_m instead of an FP64
+// division; the sum is rounded to FP32 for the region-C evaluator.
 __device__ __forceinline__ double c916_sig1_tab(double y, const double *__restrict__ e) {
   const double a = (double)HK_A916_F;
   const double y2 = y * y;
@@ -447,7 +455,7 @@ __device__ __forceinline__ double c916_sig1_tab(double y, const double *__restri
 #pragma unroll 4
   for (int m = 1; m <= HK_SIG1_M; ++m) {
     const double am2 = a * a * m * m;
-    s = __fma_rn(e[m - 1], __drcp_rn(am2 + y2), s);
+    s = __fma_rn(e[m - 1], rcp_d(am2 + y2), s);
   }
   return s;
 }

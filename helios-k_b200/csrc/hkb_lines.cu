@@ -100,8 +100,19 @@ cudaError_t sort_lines_by_nu(int64_t n, double *nu_d, int64_t *order_d,
 // power-of-two scale of the mixed form's FP32 sums.  wbits holds two words
 // per state: {half-width bits, term bits} (both non-negative doubles, so
 // their bit patterns order like the values).
+// Threads per CTA of the line prep, 4 CTAs per SM: ~1500 instructions per line
+// (a third FP64), about 100 registers.  1e7 lines of one state: 1.15 ms with the
+// window searches out of line, 0.76 ms with their estimates tried inline (20
+// warps per SM at 96 registers spill: 0.81 ms); 1.12 GB of records and 0.4 GB
+// of columns would take 0.23 ms.  Bound: issue and FP64 latency at 16 warps.
+constexpr int PREP_THREADS = 128;
+static unsigned prep_blocks(int64_t n) {
+  const int64_t nb = (n + PREP_THREADS - 1) / PREP_THREADS;
+  return (unsigned)(nb < 4736 ? nb : 4736);
+}
+
 template <bool MIXED, int MODE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(PREP_THREADS, 4)
 line_prep_kernel(LinesDev L, GridDev g, const StateDev *__restrict__ states,
                  void *__restrict__ out, unsigned long long *__restrict__ wbits) {
   const int s = blockIdx.y;
@@ -149,8 +160,8 @@ count_pairs_kernel(LinesDev L, GridDev g, const StateDev *__restrict__ st,
   for (int64_t l = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; l < L.n;
        l += (int64_t)gridDim.x * blockDim.x) {
     const LineState ls = prep_line(L, *st, l);
-    int64_t w[6];
-    line_windows(g, *st, ls, 0, g.nx, w);
+    int w[6];
+    line_windows(g, *st, ls, 0, (int)g.nx, w);
     a += (unsigned long long)((w[1] - w[0]) + (w[5] - w[4]));
     b += (unsigned long long)((w[2] - w[1]) + (w[4] - w[3]));
     c += (unsigned long long)(w[3] - w[2]);
@@ -193,13 +204,11 @@ cudaError_t launch_line_prep(bool mixed, const LinesDev &L, const GridDev &g, St
   cudaError_t e = cudaMemsetAsync(wbits_d, 0, 2 * nstates * sizeof(unsigned long long), stream);
   if (e != cudaSuccess) return e;
   if (L.n > 0) {
-    const int64_t nb = (L.n + 255) / 256;
-    const int bx = (int)(nb < 2368 ? nb : 2368);
-    dim3 grid(bx, nstates);
+    dim3 grid(prep_blocks(L.n), nstates);
     if (mixed)
-      line_prep_kernel<true, PREP_ALL><<<grid, 256, 0, stream>>>(L, g, states_d, prep_d, wbits_d);
+      line_prep_kernel<true, PREP_ALL><<<grid, PREP_THREADS, 0, stream>>>(L, g, states_d, prep_d, wbits_d);
     else
-      line_prep_kernel<false, PREP_ALL><<<grid, 256, 0, stream>>>(L, g, states_d, prep_d, wbits_d);
+      line_prep_kernel<false, PREP_ALL><<<grid, PREP_THREADS, 0, stream>>>(L, g, states_d, prep_d, wbits_d);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -213,9 +222,8 @@ cudaError_t launch_state_stats(const LinesDev &L, const GridDev &g, StateDev *st
   cudaError_t e = cudaMemsetAsync(wbits_d, 0, 2 * nstates * sizeof(unsigned long long), stream);
   if (e != cudaSuccess) return e;
   if (L.n > 0) {
-    const int64_t nb = (L.n + 255) / 256;
-    dim3 grid((unsigned)(nb < 2368 ? nb : 2368), nstates);
-    line_prep_kernel<true, PREP_STATS><<<grid, 256, 0, stream>>>(L, g, states_d, nullptr, wbits_d);
+    dim3 grid(prep_blocks(L.n), nstates);
+    line_prep_kernel<true, PREP_STATS><<<grid, PREP_THREADS, 0, stream>>>(L, g, states_d, nullptr, wbits_d);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -226,12 +234,11 @@ cudaError_t launch_state_stats(const LinesDev &L, const GridDev &g, StateDev *st
 cudaError_t launch_line_records(bool mixed, const LinesDev &L, const GridDev &g,
                                 const StateDev *state_d, void *prep_d, cudaStream_t stream) {
   if (L.n == 0) return cudaSuccess;
-  const int64_t nb = (L.n + 255) / 256;
-  dim3 grid((unsigned)(nb < 2368 ? nb : 2368), 1);
+  dim3 grid(prep_blocks(L.n), 1);
   if (mixed)
-    line_prep_kernel<true, PREP_RECORDS><<<grid, 256, 0, stream>>>(L, g, state_d, prep_d, nullptr);
+    line_prep_kernel<true, PREP_RECORDS><<<grid, PREP_THREADS, 0, stream>>>(L, g, state_d, prep_d, nullptr);
   else
-    line_prep_kernel<false, PREP_RECORDS><<<grid, 256, 0, stream>>>(L, g, state_d, prep_d, nullptr);
+    line_prep_kernel<false, PREP_RECORDS><<<grid, PREP_THREADS, 0, stream>>>(L, g, state_d, prep_d, nullptr);
   return cudaGetLastError();
 }
 
@@ -268,8 +275,8 @@ __global__ void prep_dump_kernel(LinesDev L, GridDev g, StateDev st,
   out4[4 * l + 1] = ls.S;
   out4[4 * l + 2] = ls.iad;
   out4[4 * l + 3] = ls.vy;
-  int64_t w[6];
-  line_windows(g, st, ls, 0, g.nx, w);
+  int w[6];
+  line_windows(g, st, ls, 0, (int)g.nx, w);
   for (int k = 0; k < 6; ++k) win6[6 * l + k] = w[k];
 }
 

@@ -30,8 +30,8 @@ __device__ __forceinline__ void prep_record(const LinesDev &L, const GridDev &g,
                                             int64_t l, const double *__restrict__ e916,
                                             void *__restrict__ out, double &w_loc, double &s1_loc) {
   const LineState ls = prep_line(L, st, l);
-  int64_t w[6];
-  line_windows(g, st, ls, 0, g.nx, w);
+  int w[6];
+  line_windows(g, st, ls, 0, (int)g.nx, w);
   // S1 per profile (S3_kernel voigt.h:452-463)
   const double Sc = ls.S * (1.0 / 1.7724538509055160273);
   const double S1 = g.profile <= 2 ? ls.S * ls.vy / CUDART_PI : (g.profile == 3 ? Sc : ls.S);
@@ -107,22 +107,23 @@ __device__ __forceinline__ void prep_record(const LinesDev &L, const GridDev &g,
     // region C's Algorithm-916 part: |x| < sqrt(36 - y^2), from the FP64
     // offsets (a point within rounding of r = 6 may fall on either side;
     // both evaluators hold there)
-    int64_t t0 = w[3], t1 = w[3];
+    int t0 = w[3], t1 = w[3];
     if (w[3] > w[2] && Y < 36.0) {
       const double xt = sqrt(36.0 - Y);
       const double x0 = (g.numin - ls.nu) * ls.iad, vb = g.dnu * ls.iad;
-      const double k0 = floor((-xt - x0) / vb) + 1.0, k1 = floor((xt - x0) / vb) + 1.0;
-      t0 = (int64_t)fmin(fmax(k0, (double)w[2]), (double)w[3]);
-      t1 = (int64_t)fmin(fmax(k1, (double)t0), (double)w[3]);
+      const double ivb = 1.0 / vb;
+      const double k0 = floor((-xt - x0) * ivb) + 1.0, k1 = floor((xt - x0) * ivb) + 1.0;
+      t0 = (int)fmin(fmax(k0, (double)w[2]), (double)w[3]);
+      t1 = (int)fmin(fmax(k1, (double)t0), (double)w[3]);
     }
-    r.t0 = (int)t0;
-    r.t1 = (int)t1;
-    r.i0 = (int)w[0];
-    r.b0 = (int)w[1];
-    r.c0 = (int)w[2];
-    r.c1 = (int)w[3];
-    r.b1 = (int)w[4];
-    r.i1 = (int)w[5];
+    r.t0 = t0;
+    r.t1 = t1;
+    r.i0 = w[0];
+    r.b0 = w[1];
+    r.c0 = w[2];
+    r.c1 = w[3];
+    r.b1 = w[4];
+    r.i1 = w[5];
     reinterpret_cast<LinePrepF *>(out)[l] = r;
   } else {
     const double ey = hasC ? erfcx(ls.vy) : 1.0;
@@ -135,12 +136,12 @@ __device__ __forceinline__ void prep_record(const LinesDev &L, const GridDev &g,
     r.Sc = Sc;
     r.ey = ey;
     r.sig1 = sig1;
-    r.i0 = (int)w[0];
-    r.b0 = (int)w[1];
-    r.c0 = (int)w[2];
-    r.c1 = (int)w[3];
-    r.b1 = (int)w[4];
-    r.i1 = (int)w[5];
+    r.i0 = w[0];
+    r.b0 = w[1];
+    r.c0 = w[2];
+    r.c1 = w[3];
+    r.b1 = w[4];
+    r.i1 = w[5];
     r.dsig1 = hasC ? (float)c916_dsig1_tab(ls.vy, e916) : 0.f;
     r.plinth = (g.plinth && w[5] > w[0]) ? plinth_d(g, S1, Sc, ls.iad, ls.vy) : 0.0;
     reinterpret_cast<LinePrep *>(out)[l] = r;
