@@ -784,8 +784,10 @@ cudaError_t launch_opacity_vjp(bool mixed, const LinesDev &L, const GridDev &g,
                                double *G_d, const int64_t *order_d, double *dlogS_d,
                                double *dgam_d, int log_gamma, double *dTP_d, cudaStream_t stream) {
   mixed = mixed && g.profile <= 2;  // Doppler and binned Gaussian: the FP64 form
-  cudaError_t e = cudaMemsetAsync(G_d, 0, 4 * sizeof(double) * (size_t)L.n, stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(dTP_d, 0, 2 * sizeof(double), stream);
+  // (the two scalars follow the sums of a non-empty list: one memset)
+  const bool tail = dTP_d == G_d + 4 * L.n;
+  cudaError_t e = cudaMemsetAsync(G_d, 0, (4 * (size_t)L.n + (tail ? 2 : 0)) * sizeof(double), stream);
+  if (e == cudaSuccess && !tail) e = cudaMemsetAsync(dTP_d, 0, 2 * sizeof(double), stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(ticket_d, 0, sizeof(unsigned), stream);
   if (e != cudaSuccess) return e;
   if (L.n == 0 || g.nx == 0) return cudaSuccess;

@@ -66,6 +66,7 @@ struct hk_ctx {
   DevBuf states, ticket, wbits, Kwork, outwork, scratch, prep;
   DevBuf vpart, vcnt;  // split-tile partial sums and per-tile counters
   DevBuf sscale, gscale, adjwork;  // per-line scales (adjoint parameters), VJP workspace
+  DevBuf scalebad;                 // the device check's two words of those scales
   size_t prep_budget = (size_t)24 << 30;  // bytes of per-(state, line) records per batch
   size_t part_budget = (size_t)4 << 30;   // bytes of split-tile partial sums per batch
   double voigt_ms_acc = 0.0;
@@ -166,7 +167,7 @@ void hk_destroy(hk_ctx *c) {
   for (DevBuf *b : {&c->nu0, &c->Sfile, &c->EL, &c->gam, &c->nexp, &c->delta,
                     &c->Aterm, &c->iso, &c->order, &c->states, &c->ticket,
                     &c->prep, &c->wbits, &c->Kwork, &c->outwork, &c->scratch,
-                    &c->qrV, &c->qrC, &c->qrD, &c->vpart, &c->vcnt, &c->sscale, &c->gscale, &c->adjwork,
+                    &c->qrV, &c->qrC, &c->qrD, &c->vpart, &c->vcnt, &c->sscale, &c->gscale, &c->scalebad, &c->adjwork,
                     &c->tunework, &c->meanwork, &c->cia_nu, &c->cia_val, &c->cia_tab})
     b->release();
   for (auto &e : c->ev)
@@ -1068,29 +1069,34 @@ hk_status hk_set_line_scales_device(hk_ctx *c, const double *s_scale, const doub
   const int64_t n = c->nlines;
   DevBuf *dst[2] = {&c->sscale, &c->gscale};
   const double **field[2] = {&c->L.sscale, &c->L.gscale};
+  auto restore = [&](int q) {
+    dst[q]->release();
+    *field[q] = nullptr;
+  };
   for (int q = 0; q < 2; ++q) {
-    if (!src[q]) {
-      dst[q]->release();
-      *field[q] = nullptr;
-      continue;
-    }
-    // the values, then the word of the first invalid load index
-    CUDA_TRY(c, dst[q]->ensure(n * sizeof(double) + sizeof(unsigned long long)));
-    unsigned long long *bad = reinterpret_cast<unsigned long long *>(dst[q]->as<double>() + n);
-    CUDA_TRY(c, launch_gather_scales(n, c->order.as<int64_t>(), src[q], dst[q]->as<double>(), bad, s));
-    unsigned long long first_bad = 0;
-    CUDA_TRY(c, cudaMemcpyAsync(&first_bad, bad, sizeof first_bad, cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(c, cudaStreamSynchronize(s));
-    if (first_bad < (unsigned long long)n) {
-      // the buffer now holds the invalid values: no multiplier stays in force
-      for (int r = 0; r < 2; ++r) {
-        dst[r]->release();
-        *field[r] = nullptr;
-      }
-      return fail(c, HK_ERR_ARG, "line scale %lld must be finite and > 0", (long long)first_bad);
-    }
-    *field[q] = dst[q]->as<double>();
+    if (src[q]) CUDA_TRY(c, dst[q]->ensure(n * sizeof(double)));
+    else restore(q);
   }
+  if (!src[0] && !src[1]) {
+    ok(c);
+    return HK_OK;
+  }
+  // both arrays in one launch, and one 16-byte read of the check's words
+  CUDA_TRY(c, c->scalebad.ensure(2 * sizeof(unsigned long long)));
+  CUDA_TRY(c, launch_gather_scales(n, c->order.as<int64_t>(), src[0], dst[0]->as<double>(), src[1],
+                                   dst[1]->as<double>(), c->scalebad.as<unsigned long long>(), s));
+  unsigned long long bad[2] = {0, 0};
+  CUDA_TRY(c, cudaMemcpyAsync(bad, c->scalebad.p, sizeof bad, cudaMemcpyDeviceToHost, s));
+  CUDA_TRY(c, cudaStreamSynchronize(s));
+  for (int q = 0; q < 2; ++q)
+    if (src[q] && bad[q] < (unsigned long long)n) {
+      // the buffer now holds the invalid values: no multiplier stays in force
+      restore(0);
+      restore(1);
+      return fail(c, HK_ERR_ARG, "line scale %lld must be finite and > 0", (long long)bad[q]);
+    }
+  for (int q = 0; q < 2; ++q)
+    if (src[q]) *field[q] = dst[q]->as<double>();
   ok(c);
   return HK_OK;
 }
@@ -1122,9 +1128,6 @@ static hk_status opacity_vjp(hk_ctx *c, double T, double P, int precision, const
   // the plain per-line records (FP64 windows and constants) of this state
   CUDA_TRY(c, launch_line_prep(false, c->L, c->g, c->states.as<StateDev>(), 1, c->prep.p,
                                c->wbits.as<unsigned long long>(), true, s));
-  // the device copy of the state (wmax finalised) drives both passes
-  CUDA_TRY(c, cudaMemcpyAsync(hs.data(), c->states.p, sizeof(StateDev), cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(c, cudaStreamSynchronize(s));
   const double *ud = u;
   size_t need = 4 * (size_t)std::max<int64_t>(n, 1) + 2;
   if (!u_on_device) need += (size_t)nx;

@@ -42,26 +42,37 @@ cudaError_t launch_gather_lines(int64_t n, const int64_t *order_d,
 }
 
 // Per-line multipliers from load order into the nu-sorted order, dst[k] =
-// src[order[k]], each checked to be finite and > 0: *bad ends as the
-// smallest load index of a value that is not (n when all are).
-__global__ void bad_init_kernel(unsigned long long *bad, int64_t n) { *bad = (unsigned long long)n; }
-
+// src[order[k]], strengths (q = 0) and widths (q = 1; either may be null) in one
+// launch, each checked to be finite and > 0: bad[q] ends as the smallest load
+// index of a value that is not (all ones when all are).
 __global__ void gather_scales_kernel(int64_t n, const int64_t *__restrict__ order,
-                                     const double *__restrict__ src, double *__restrict__ dst,
+                                     const double *__restrict__ s_src, double *__restrict__ s_dst,
+                                     const double *__restrict__ g_src, double *__restrict__ g_dst,
                                      unsigned long long *bad) {
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n;
        k += (int64_t)gridDim.x * blockDim.x) {
     const int64_t j = order[k];
-    const double v = src[j];
-    dst[k] = v;
-    if (!(v > 0.0 && v <= 1.7976931348623157e308)) atomicMin(bad, (unsigned long long)j);
+    if (s_src) {
+      const double v = s_src[j];
+      s_dst[k] = v;
+      if (!(v > 0.0 && v <= 1.7976931348623157e308)) atomicMin(bad, (unsigned long long)j);
+    }
+    if (g_src) {
+      const double v = g_src[j];
+      g_dst[k] = v;
+      if (!(v > 0.0 && v <= 1.7976931348623157e308)) atomicMin(bad + 1, (unsigned long long)j);
+    }
   }
 }
 
-cudaError_t launch_gather_scales(int64_t n, const int64_t *order_d, const double *src_d,
-                                 double *dst_d, unsigned long long *bad_d, cudaStream_t stream) {
-  bad_init_kernel<<<1, 1, 0, stream>>>(bad_d, n);
-  if (n > 0) gather_scales_kernel<<<1184, 256, 0, stream>>>(n, order_d, src_d, dst_d, bad_d);
+cudaError_t launch_gather_scales(int64_t n, const int64_t *order_d, const double *s_src, double *s_dst,
+                                 const double *g_src, double *g_dst, unsigned long long *bad_d,
+                                 cudaStream_t stream) {
+  const cudaError_t e = cudaMemsetAsync(bad_d, 0xff, 2 * sizeof(unsigned long long), stream);
+  if (e != cudaSuccess || n == 0) return e;
+  const int64_t nb = (n + 255) / 256;
+  gather_scales_kernel<<<(unsigned)(nb < 1184 ? nb : 1184), 256, 0, stream>>>(n, order_d, s_src, s_dst, g_src,
+                                                                             g_dst, bad_d);
   return cudaGetLastError();
 }
 
