@@ -1009,6 +1009,41 @@ __device__ __forceinline__ void sweep_G(const RecF &r, int wb, int lane,
   }
 }
 
+// Plinth removal, a whole slice in one of regions A and B (INB): the terms of
+// sweep_G with its operations in its order (same bits), two points to a packed
+// instruction and no test per point.  FACT: the edge lies in the same region
+// (factored difference), else term - plinth.  kd: the lane's first tile point.
+template <bool INB, bool FACT, int PPL>
+__device__ __forceinline__ void sweep_PL(const RecF &rr, const ExtPL &pe, double kd,
+                                         const float2 (&kf)[PPL / 2], float2 (&a32)[PPL / 2]) {
+  const CoefB c = load_coef(rr);
+  const float2 Y = dup(rr.y * rr.y);
+  const double vbd = pe.vb, D0 = pe.D0, xd = pe.xd;
+  const float2 xcf = dup(pe.xcf), ic = dup(pe.ic), nplf = dup(-pe.plf);
+  const float2 q2 = dup(pe.q2), q1 = dup(pe.q1), q0 = dup(pe.q0);
+#pragma unroll
+  for (int q = 0; q < PPL / 2; ++q) {
+    const float2 x = x_pair(c, kf[q]);
+    const float2 s = __fmul2_rn(x, x);
+    float2 num = c.S1f, inv;
+    if (INB) {
+      gh2_pair(c, s, num, inv);
+    } else {
+      const float2 u = __ffma2_rn(x, x, Y);
+      inv = make_float2(rcp_fast(u.x), rcp_fast(u.y));
+    }
+    if (FACT) {
+      const float2 dx = make_float2((float)(xd - fabs(fma(kd + 64.0 * q, vbd, D0))),
+                                    (float)(xd - fabs(fma(kd + (64.0 * q + 32.0), vbd, D0))));
+      float2 w = __fmul2_rn(__fmul2_rn(dx, __fadd2_rn(xcf, make_float2(fabsf(x.x), fabsf(x.y)))), ic);
+      if (INB) w = __fmul2_rn(w, __ffma2_rn(__ffma2_rn(q2, s, q1), s, q0));
+      a32[q] = __fadd2_rn(a32[q], __fmul2_rn(__fmul2_rn(c.S1f, inv), w));
+    } else {
+      a32[q] = __fadd2_rn(a32[q], __ffma2_rn(num, inv, nplf));
+    }
+  }
+}
+
 // Plinth removal, a line summed per point in FP64 (HK_F_PL64: its cut edge
 // lies in region C or close to a region boundary, or FP32 cannot hold it):
 // the FP64 form's terms (regions C, B, A) less the plinth, from the line's
@@ -1322,6 +1357,18 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t
               const int b = __ffs(mX) - 1;
               mX &= mX - 1;
               const ExtPL *pe = ext_pl + g32 + b;
+              const int plc = rf[g32 + b].flags & (HK_F_PLA | HK_F_PLB);
+              if ((bA >> b) & 1u) {
+                // (every line in its place of the group's order)
+                if (plc == HK_F_PLA) sweep_PL<false, true, PPL>(rf[g32 + b], *pe, (double)(wb + lane), kf, a32);
+                else sweep_PL<false, false, PPL>(rf[g32 + b], *pe, (double)(wb + lane), kf, a32);
+                continue;
+              }
+              if ((bB >> b) & 1u) {
+                if (plc == HK_F_PLB) sweep_PL<true, true, PPL>(rf[g32 + b], *pe, (double)(wb + lane), kf, a32);
+                else sweep_PL<true, false, PPL>(rf[g32 + b], *pe, (double)(wb + lane), kf, a32);
+                continue;
+              }
               sweep_G<false, false, PPL, EXT>(rf[g32 + b], wb, lane, kf, a32, cacc, g.profile, nullptr, 0.f,
                                               pe);
               sweep_C<SL, EXT>(rf[g32 + b], Rtab + (g32 + b) * HK_C916_MR, cacc, wb, lane, nullptr, 0.f,
