@@ -116,7 +116,8 @@ __device__ __forceinline__ double gauss_vb(const RecF &r) { return reinterpret_c
 // flags: HK_F_WEAK -- level above HK_MAX_LEVEL (2^768 below the strongest
 // line) or HK_PF_RANGE: the line is summed in FP64 with S1f = 1;
 // HK_F_WIDE -- some x^2 + Y in the window reaches 1e18, so two region-A
-// denominators may not be multiplied in FP32 (paired reciprocals are off);
+// denominators may not be multiplied in FP32 (its region A takes sweep_G, a
+// reciprocal per point);
 // with plinth removal, HK_F_PLA / HK_F_PLB -- the cut edge x_c lies in
 // region A / B, whose points take the factored difference t(x) - t(x_c);
 // HK_F_PL64 -- the line is summed per point in FP64 (HK_PF_PL64).
@@ -219,6 +220,16 @@ __device__ __forceinline__ float2 f2(double v) {
 // chunk -- its strength level (0..HK_MAX_LEVEL), HK_MAX_LEVEL + 1 for lines
 // summed in FP64 (weak), HK_MAX_LEVEL + 2 for lines without points in the
 // tile -- and stage_mixed builds the record for that key.
+// v 2^e as ldexp gives it, |e| <= 2000.  A product of three: ldexp's code and
+// branches sat in the level flushes and in the staging, and this kernel pays
+// for code size (64 registers, several thousand instructions, "no instruction"
+// stalls): 24-state table 14.67 -> 13.56 ms, 4 ExoMol states 19.18 -> 18.63, 1e5
+// lines x 3e6 points with the fit 724 -> 683 us.
+__device__ __forceinline__ double scale2_d(double v, int e) {
+  const int h = e >> 1;
+  return v * __hiloint2double((1023 + h) << 20, 0) * __hiloint2double((1023 + e - h) << 20, 0);
+}
+
 // Record loads: the Voigt launch reads records another kernel wrote (the
 // read-only path is fine); the fused table kernel reads records its own CTAs
 // wrote into reused ring slots, so its loads go to L2 (.cg), never through
@@ -376,7 +387,7 @@ __device__ __forceinline__ void stage_mixed(const LinePrepF *__restrict__ P, con
   // the tile point nearest the centre (|kc| <= 2^23 keeps k - kc exact)
   const double kc = fmin(fmax(rint(-D0 / vb), -8388608.0), 8388608.0);
   // S1f = S1 * 2^(s1exp + 96 lev): the line's largest term near 2^40
-  const double S1f = weak ? 1.0 : ldexp(lp.S1, s1exp + HK_LEVEL_BITS * lev);
+  const double S1f = weak ? 1.0 : scale2_d(lp.S1, s1exp + HK_LEVEL_BITS * lev);
   r.S1f = (float)S1f;
   r.C1 = (float)(S1f * (double)lp.A1);
   r.C0 = (float)(S1f * (double)lp.B1);
@@ -509,7 +520,8 @@ __device__ __forceinline__ void stage_plain(const LinePrep *__restrict__ P, cons
 //   HK_CLS_BM  [lo, hi) lies in region B or C (window edge in the slice, or
 //              region C in it);
 //   HK_CLS_AM  [lo, hi) lies in region A (window edge in the slice);
-//   HK_CLS_G   [lo, hi) holds an A/B region boundary;
+//   HK_CLS_G   [lo, hi) holds an A/B region boundary (or region A of a line with
+//              HK_F_WIDE, whose denominators may not be paired);
 //   HK_CLS_W   an HK_F_WEAK line (FP64 sums);
 //   HK_CLS_BF, HK_CLS_AF  as B and A but for far-field blocks of the slice,
 //              which they skip;
@@ -577,7 +589,7 @@ __device__ __forceinline__ void far_terms(const RecF &r, int blo, float (&fq)[HK
 __device__ __forceinline__ void far_flush(float (&fq)[HK_FN], double *__restrict__ fdw, int lane,
                                           int nblk, int s1exp, int lev) {
   if (lane < nblk) {
-    const double u = ldexp(1.0, -(s1exp + HK_LEVEL_BITS * lev));
+    const double u = scale2_d(1.0, -(s1exp + HK_LEVEL_BITS * lev));
 #pragma unroll
     for (int n = 0; n < HK_FN; ++n) fdw[n * nblk + lane] = fma((double)fq[n], u, fdw[n * nblk + lane]);
   }
@@ -586,7 +598,7 @@ __device__ __forceinline__ void far_flush(float (&fq)[HK_FN], double *__restrict
 }
 
 // fm: the slice's far blocks (FAR), which the direct sweeps skip
-template <int SLICE, bool FAR = false>
+template <int SLICE, bool FAR = false, bool WG = false>
 __device__ __forceinline__ int classify(const RecF &r, int wb, unsigned &fm) {
   fm = 0u;
   const int we = wb + SLICE;
@@ -600,7 +612,8 @@ __device__ __forceinline__ int classify(const RecF &r, int wb, unsigned &fm) {
   const bool full = lo == wb && hi == we;
   const bool noC = r.c0 >= r.c1 || r.c1 <= lo || r.c0 >= hi;
   if (r.b0 <= lo && r.b1 >= hi) return (full && noC) ? (fm ? HK_CLS_BF : HK_CLS_B) : HK_CLS_BM;
-  if (r.b0 >= r.b1 || r.b1 <= lo || r.b0 >= hi) return full ? (fm ? HK_CLS_AF : HK_CLS_A) : HK_CLS_AM;
+  if ((r.b0 >= r.b1 || r.b1 <= lo || r.b0 >= hi) && !(WG && (r.flags & HK_F_WIDE)))
+    return full ? (fm ? HK_CLS_AF : HK_CLS_A) : HK_CLS_AM;
   return HK_CLS_G;
 }
 
@@ -769,7 +782,6 @@ __device__ __forceinline__ void sweep_A(const RecF &rr, int wb, int lane,
   const CoefB c = load_coef(rr);
   const float Yf = rr.y * rr.y;
   const float2 Y = make_float2(Yf, Yf);
-  const bool wide = rr.flags & HK_F_WIDE;
   const int lo = max(rr.i0, wb), hi = min(rr.i1, wb + 32 * PPL);
 #pragma unroll
   for (int q = 0; q < PPL / 2; ++q) {
@@ -789,7 +801,7 @@ __device__ __forceinline__ void sweep_A(const RecF &rr, int wb, int lane,
       u.x = m0 ? u.x : 1e6f;
       u.y = m1 ? u.y : 1e6f;
     }
-    float2 inv = wide ? make_float2(rcp_fast(u.x), rcp_fast(u.y)) : rcp_pair(u);
+    float2 inv = rcp_pair(u);
     if (AM) {
       inv.x = m0 ? inv.x : 0.f;
       inv.y = m1 ? inv.y : 0.f;
@@ -1161,7 +1173,7 @@ __device__ __forceinline__ void sweep_plain(const RecD &r, int wb, int lane,
 template <int PPL>
 __device__ __forceinline__ void flush_sums(float2 (&a32)[PPL / 2], double *__restrict__ cacc,
                                            int wb, int lane, int s1exp, int lev) {
-  const double u = ldexp(1.0, -(s1exp + HK_LEVEL_BITS * lev));
+  const double u = scale2_d(1.0, -(s1exp + HK_LEVEL_BITS * lev));
 #pragma unroll
   for (int p = 0; p < PPL; ++p) {
     const int k = wb + lane + 32 * p;
@@ -1290,17 +1302,18 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t
       const int64_t l = L0 + c + (int64_t)tid * nch;
       if (tid < cnt_c) key = line_key<CG>(PF, l, g0, g1, s1exp);
       if (tid < CH) {
-        const unsigned lt = (1u << lane) - 1u;
-#pragma unroll
-        for (int v = 0; v < HK_NKEY; ++v) {
-          const unsigned m = __ballot_sync(0xffffffffu, key == v);
-          if (key == v) rank = __popc(m & lt);
-          if (lane == 0) s_kcnt[warp][v] = __popc(m);
-        }
+        // one match and one store per distinct key instead of a ballot per key
+        // (24-state table 13.41 -> 13.21 ms); key HK_NKEY: no line, not counted
+        if (lane < HK_NKEY) s_kcnt[warp][lane] = 0;
+        __syncwarp();
+        const unsigned m = __match_any_sync(0xffffffffu, key);
+        rank = __popc(m & ((1u << lane) - 1u));
+        if (rank == 0 && key < HK_NKEY) s_kcnt[warp][key] = __popc(m);
       }
       __syncthreads();
       if (tid < cnt_c) {
         int pos = rank;
+#pragma unroll 1
         for (int v = 0; v < key; ++v)
 #pragma unroll
           for (int w = 0; w < CH / 32; ++w) pos += s_kcnt[w][v];
@@ -1321,7 +1334,7 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t
       for (int g32 = 0; g32 < cnt_c; g32 += 32) {
         const int j = g32 + lane;
         unsigned fm = 0u;  // the line's far blocks in this slice
-        const int cls = (j < cnt_c) ? classify<SLICE, FAR>(rf[j], ws, fm) : HK_CLS_SKIP;
+        const int cls = (j < cnt_c) ? classify<SLICE, FAR, !G34>(rf[j], ws, fm) : HK_CLS_SKIP;
         if (SUB > 1) fm >>= (wb - ws) / HK_FB;  // the warp's own blocks
         const int lev = (j < cnt_c) ? (rf[j].flags >> 8) : 0;
         const unsigned bB = __ballot_sync(0xffffffffu, cls == HK_CLS_B);
@@ -1472,19 +1485,20 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t
 #pragma unroll
         for (int n = 0; n < HK_FN; ++n) fq[n] = 0.f;
         int flev = -1;
-        for (int j = warp; j < cnt_c; j += SH::WARPS) {
-          const RecF &r = rf[j];
+        for (int j = warp;; j += SH::WARPS) {
+          const bool end = j >= cnt_c;
+          const RecF &r = rf[end ? 0 : j];
           const unsigned fmk = r.fmask;
-          if (fmk == 0u) continue;
+          if (fmk == 0u && !end) continue;
           const bool far = SUB == 1 ? (fmk >> lane) & 1u : lane < NBLK && ((fmk >> (fb0 + lane)) & 1u);
           const int lev = r.flags >> 8;
-          if (lev != flev) {
+          if (end || lev != flev) {
             if (flev >= 0) far_flush(fq, fdw, lane, NBLK, s1exp, flev);
+            if (end) break;
             flev = lev;
           }
           if (far) far_terms(r, blo, fq);
         }
-        if (flev >= 0) far_flush(fq, fdw, lane, NBLK, s1exp, flev);
       }
     } else {
       for (int j = 0; j < cnt_c; ++j)
