@@ -213,6 +213,13 @@ struct KdistArgs {
 
 constexpr uint64_t KD_KEY_END = 0xffffffffffffffffull;  // after every key of a value
 
+// 2 j / den - 1 (inv = 1 / den) with the quotient rounded as the division
+// rounds it, but for rare last bits: one residual step
+__device__ __forceinline__ double grid_pos(int j, double den, double inv) {
+  const double t = 2.0 * j, q = t * inv;
+  return __fma_rn(__fma_rn(-q, den, t), inv, q) - 1.0;
+}
+
 // findCut (resample.h:362-388) on the sorted bin: within a bin at most one
 // index j has K[j] <= kmin < K[j+1]; the empty-bin rules follow it.  s_trans
 // holds -1 and a barrier has passed.
@@ -335,16 +342,16 @@ __device__ __forceinline__ void fit_moments(const KdistArgs &a, const double *b,
   for (int k = tid + IPT * THREADS; k < n; k += THREADS) af = __fma_rn(ft[k], b[k], af);
   for (int o = 16; o > 0; o >>= 1) af += __shfl_xor_sync(0xffffffffu, af, o);
   if (lane == 0) buf[groups * KD_MG * WARPS + warp] = af;
-  const double h = 2.0 / ((double)n - 1.0);
+  const double den = (double)n - 1.0, inv = 1.0 / den;
   for (int gq = 0; gq < groups; ++gq) {
     double acc[KD_MG];
 #pragma unroll
     for (int q = 0; q < KD_MG; ++q) acc[q] = 0.0;
     for (int k = tid; k < (n + 1) / 2; k += THREADS) {
       const int k2 = n - 1 - k;
-      // (the middle point of an odd count has x = 0 to a rounding: odd T vanish)
+      // (the middle point of an odd count has x = 0: odd T vanish)
       const double bl = b[k], bh = k2 > k ? b[k2] : 0.0;
-      const double x = __fma_rn((double)k, h, -1.0), x2 = 2.0 * x, s = bl + bh, d = bl - bh;
+      const double x = grid_pos(k, den, inv), x2 = 2.0 * x, s = bl + bh, d = bl - bh;
       double ta = 1.0, tb = x;
       for (int i = 0; i < gq * KD_MG; i += 2) {
         ta = __fma_rn(x2, tb, -ta);
@@ -636,9 +643,9 @@ kdist_kernel(KdistArgs a) {
 
   // expfx_kernel (x = -1 + 2 j / Nxb) then rescale(-1): the even and odd parts
   // of the series at x give the values at x and -x = x_(Nxb - j)
-  const double h = 2.0 / (double)nxb, iu = 1.0 / a.unitScale;
+  const double inv = 1.0 / (double)nxb, iu = 1.0 / a.unitScale;
   for (int j = tid; j <= nxb / 2; j += THREADS) {
-    const double x = __fma_rn((double)j, h, -1.0), x2 = 2.0 * x;
+    const double x = grid_pos(j, (double)nxb, inv), x2 = 2.0 * x;
     double ta = 1.0, tb = x, ev = 0.0, od = 0.0;
     int i = 0;
     for (; i + 1 < nc; i += 2) {

@@ -5,8 +5,8 @@
 // writer: there are no atomics on K and no partial-row reduction (the
 // reference's 32 KS_d rows + AddKStreams_kernel, voigt.h:728-742, are gone).
 // For its tile the CTA
-//   1. finds the nu-sorted line range whose cutoff windows can reach the tile
-//      (warp-parallel lower_bound),
+//   1. takes the nu-sorted line range whose cutoff windows can reach the tile
+//      (tile_range_kernel),
 //   2. stages the lines in chunks of CH through shared memory: each thread
 //      loads one line's state record (FP64 parameters and global index
 //      windows, written by line_prep_kernel), clips the windows to the tile
