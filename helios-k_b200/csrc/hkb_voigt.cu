@@ -1625,6 +1625,9 @@ voigt_sum_kernel(const void *__restrict__ prep, const longlong2 *__restrict__ ra
     if (tid == 0) s_ticket = (int)atomicAdd(ticket, 1u);
     __syncthreads();
     const int t = s_ticket;
+    // every warp has read s_ticket before the next ticket is written to it:
+    // sum_tile may return without a barrier (a part or a tile without lines)
+    __syncthreads();
     if (t >= total_tickets) break;
     // ticket -> (tile of a state, part of that tile's line range, sub-tile)
     const int tp = t / SUB, sub = t - tp * SUB;
