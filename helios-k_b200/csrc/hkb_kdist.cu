@@ -190,13 +190,17 @@ qr_kernel(int nxb, int nc, int moments, double *__restrict__ V, double *__restri
   }
 }
 
-// Whether the fit of (nxb, nc) goes through the moments: the Chebyshev basis on
-// nxb equally spaced points is well conditioned for nc well below sqrt(nxb)
-// and, measured, for 6 nc <= nxb (condition number 3 - 7 from 120 points x 20
-// to 11000 x 30; coefficients within 6e-14 of the reflections').  Below 4
-// coefficients the reflections do not spread a non-finite value to all of
-// them, so those keep the reflections.
-static __host__ __device__ inline bool kdist_moments(int nxb, int nc) { return nc >= 4 && 6 * nc <= nxb; }
+// Whether the fit of (nxb, nc) goes through the moments.  The Chebyshev basis on
+// nxb equally spaced points degrades with nc^2 / nxb and, for few points, with
+// nc / nxb: condition number 3.2 at 120 points x 20, 7.0 at 2858 x 100, 4.1 at
+// 350 x 35 (6.1 at 10000 x 30) on this rule's edge, but 34 at 480 x 80 and 131 at
+// 600 x 100 beyond it, and the moments square it.  Inside the rule the
+// coefficients are nearer the exact fit than the reflections' (fit_moments).
+// Below 4 coefficients the reflections do not spread a non-finite value to all
+// of them, so those keep the reflections.
+static __host__ __device__ inline bool kdist_moments(int nxb, int nc) {
+  return nc >= 4 && 6 * nc <= nxb && 2 * nc * nc <= 7 * nxb;
+}
 
 struct KdistArgs {
   const double *K;       // nstates x nx, unsorted
@@ -308,6 +312,15 @@ __device__ void fit_reflections(const KdistArgs &a, double *work, const double *
 // reflections read 19 columns of V from L2 (1.5 MB per 10000-point bin) and
 // closed each with a block-wide sum.  The moments go in groups of KD_MG, each
 // running the recurrence up to its first.
+//
+// The moments are those of b - p, p the cubic through four of the sorted values
+// (x = -1, -1/2, 1/2, 1; without its T_3 for nc = 4), and p's coefficients are
+// added to the result: p lies in the span of T_0 .. T_(nc-2), which the fit gives
+// back exactly (f is orthogonal to it), and what the sums and M round is then
+// a small remainder, not b.  Largest coefficient error in 64 bits against
+// extended precision, median over spectra (reflections / moments of b / of
+// b - p): 10000 x 20 9.8e-16 / 2.8e-15 / 3.5e-16, 120 x 20 9.2e-16 / 3.2e-15 /
+// 3.8e-16, 2858 x 100 9.2e-16 / 9.1e-15 / 6.1e-16.
 // buf: (groups * KD_MG + 1) * warps doubles, then M if it fits.
 constexpr int KD_MG = 10;
 template <int THREADS, int IPT>
@@ -342,6 +355,16 @@ __device__ __forceinline__ void fit_moments(const KdistArgs &a, const double *b,
   for (int k = tid + IPT * THREADS; k < n; k += THREADS) af = __fma_rn(ft[k], b[k], af);
   for (int o = 16; o > 0; o >>= 1) af += __shfl_xor_sync(0xffffffffu, af, o);
   if (lane == 0) buf[groups * KD_MG * WARPS + warp] = af;
+  // p = sum p_j T_j
+  double p0, p1, p2, p3;
+  {
+    const int i1 = (n - 1) / 4, i2 = n - 1 - i1;
+    const double ve = b[n - 1] + b[0], vi = b[i2] + b[i1], de = b[n - 1] - b[0], di = b[i2] - b[i1];
+    p0 = (0.5 * ve + vi) * (1.0 / 3.0);
+    p1 = (de + di) * (1.0 / 3.0);
+    p2 = (ve - vi) * (1.0 / 3.0);
+    p3 = nc > 4 ? (de - 2.0 * di) * (1.0 / 6.0) : 0.0;
+  }
   const double den = (double)n - 1.0, inv = 1.0 / den;
   for (int gq = 0; gq < groups; ++gq) {
     double acc[KD_MG];
@@ -350,15 +373,28 @@ __device__ __forceinline__ void fit_moments(const KdistArgs &a, const double *b,
     for (int k = tid; k < (n + 1) / 2; k += THREADS) {
       const int k2 = n - 1 - k;
       // (the middle point of an odd count has x = 0: odd T vanish)
-      const double bl = b[k], bh = k2 > k ? b[k2] : 0.0;
-      const double x = grid_pos(k, den, inv), x2 = 2.0 * x, s = bl + bh, d = bl - bh;
-      double ta = 1.0, tb = x;
-      for (int i = 0; i < gq * KD_MG; i += 2) {
+      const bool two = k2 > k;
+      const double bl = b[k], bh = two ? b[k2] : 0.0;
+      const double x = grid_pos(k, den, inv), x2 = 2.0 * x, w = two ? -2.0 : -1.0;
+      double ta = __fma_rn(x2, x, -1.0), tb = __fma_rn(x2, ta, -x);  // T_2, T_3
+      // sum and difference of b - p at x and -x
+      const double s = __fma_rn(w, __fma_rn(p2, ta, p0), bl + bh);
+      const double d = __fma_rn(w, __fma_rn(p3, tb, p1 * x), bl - bh);
+      if (gq == 0) {
+        acc[0] += s;
+        acc[1] = __fma_rn(x, d, acc[1]);
+      } else {
+        for (int i = 2; i < gq * KD_MG; i += 2) {
+          ta = __fma_rn(x2, tb, -ta);
+          tb = __fma_rn(x2, ta, -tb);
+        }
+        acc[0] = __fma_rn(ta, s, acc[0]);
+        acc[1] = __fma_rn(tb, d, acc[1]);
         ta = __fma_rn(x2, tb, -ta);
         tb = __fma_rn(x2, ta, -tb);
       }
 #pragma unroll
-      for (int q = 0; q < KD_MG; q += 2) {
+      for (int q = 2; q < KD_MG; q += 2) {
         acc[q] = __fma_rn(ta, s, acc[q]);
         acc[q + 1] = __fma_rn(tb, d, acc[q + 1]);
         ta = __fma_rn(x2, tb, -ta);
@@ -398,7 +434,8 @@ __device__ __forceinline__ void fit_moments(const KdistArgs &a, const double *b,
       for (int j = 0; j < nc; ++j)
         c = __fma_rn(j == nm && tid == nm ? 1.0 / s_d[nm] : a.V[tid + (int64_t)n * j], s_z[j], c);
     }
-    // a non-finite b (its sum is m_0) leaves no coefficient finite
+    c += tid == 0 ? p0 : tid == 1 ? p1 : tid == 2 ? p2 : tid == 3 ? p3 : 0.0;
+    // a non-finite b (m_0 sums b - p) leaves no coefficient finite
     if (!isfinite(s_z[0])) c = __longlong_as_double(0x7ff8000000000000ll);
     co[tid] = c;
     s_c[tid] = c;
