@@ -841,21 +841,21 @@ cudaError_t launch_kdist(const double *K_d, int64_t k_stride, int nstates,
     kfn<<<grid, threads, dyn, stream>>>(a);
     return cudaGetLastError();
   };
-  // 1024 threads share an SM: the smallest CTA that holds the bin at 12 keys a
-  // thread lets the barriers of one bin hide behind another's work; with
-  // fewer bins than SMs a wider CTA finishes its bin sooner
-  const int64_t ctas = (int64_t)nbins * nstates;
-  const int thr = (nxb > 6144 || ctas <= 148) ? 1024 : (nxb > 3072 || ctas <= 296) ? 512 : 256;
+  // The smallest CTA that holds the bin at 12 keys a thread: 1024 threads
+  // share an SM, so the barriers of one bin hide behind another's work (20
+  // coefficients, 3000 points: 3000 bins 191 us in 256 threads, 241 in 512, 346
+  // in 1024; 6000 points 395 in 512, 498 in 1024).  With fewer bins than SMs a
+  // wider one would finish sooner (3000 points 26 us in 512 against 31, 6000
+  // 33 in 1024 against 37), but the sums' order, and so the last bits of the
+  // coefficients, goes with the width: it depends on nxb alone, and a state
+  // keeps its coefficients whatever it is fitted with and wherever.
+  const int thr = nxb > 6144 ? 1024 : nxb > 3072 ? 512 : 256;
   const int ipt = (nxb + thr - 1) / thr;
 #define KD_CASE(T, I) \
   if (thr == T && ipt <= I) return run(kdist_kernel<T, I>, T, I);
-  KD_CASE(1024, 2)
-  KD_CASE(1024, 4)
-  KD_CASE(1024, 6)
   KD_CASE(1024, 8)
   KD_CASE(1024, 10)
   KD_CASE(1024, 12)
-  KD_CASE(512, 4)
   KD_CASE(512, 8)
   KD_CASE(512, 10)
   KD_CASE(512, 12)
