@@ -473,8 +473,15 @@ __device__ __forceinline__ bool prefix_sort(const uint64_t (&v)[IPT], int n, uin
   const int e0 = warp * 32 * IPT + lane;
   auto in = [&](int i) { return e0 + 32 * i < n && !(nfloor > 0 && v[i] == floor); };
   unsigned at_[IPT];
+  // (the first key of every thread finds most crowded bins: the atomics of a
+  // crowd are taken in turn.  480 bins of 10000 points in one crowd, sort alone:
+  // 188 us without this look, 168 with it, 172 by the merge sort at once)
+  at_[0] = in(0) ? atomicAdd(cnt + prefix32(v[0], mn, sh), 1u) : 0u;
+  if (at_[0] >= KD_RUN) *s_long = 1;
+  __syncthreads();
+  if (*s_long) return false;
 #pragma unroll
-  for (int i = 0; i < IPT; ++i) at_[i] = in(i) ? atomicAdd(cnt + prefix32(v[i], mn, sh), 1u) : 0u;
+  for (int i = 1; i < IPT; ++i) at_[i] = in(i) ? atomicAdd(cnt + prefix32(v[i], mn, sh), 1u) : 0u;
   __syncthreads();
   uint4 c[KD_STEPS / 4];
   unsigned sum = 0, most = 0;
@@ -572,11 +579,11 @@ __device__ __noinline__ void merge_sort(const double *__restrict__ src, int n, v
 // step and within each step.  A bin whose values crowd into few steps takes a
 // block merge sort in registers.
 // Measured, 480 bins of 10000 points (block merge sort and reflections ->
-// this): sort alone 168 -> 93 - 118 us (173 -> 189 for bins that fall back);
-// with the fit 404 -> 149 - 174; with sorted values and reconstruction written
-// 476 -> 189 - 212.  Bound: latency, one 1024-thread CTA per SM in phases
-// between barriers (load 8 %, sort 35 %, ln 10 %, moments 25 %, reconstruction
-// 16 % of a bin's time); its 115 MB of traffic would take 18 us.
+// this): sort alone 173 -> 90 us (172 -> 168 for bins that fall back); with
+// sorted values, fit of 20 coefficients and reconstruction written 482 -> 185.
+// Bound: latency, one 1024-thread CTA per SM in phases between barriers (load
+// 8 %, sort 35 %, ln 10 %, moments 25 %, reconstruction 16 % of a bin's time);
+// its 115 MB of traffic would take 18 us.
 template <int THREADS, int IPT>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 kdist_kernel(KdistArgs a) {
