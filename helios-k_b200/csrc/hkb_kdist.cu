@@ -34,19 +34,7 @@ __device__ __forceinline__ double key2f(uint64_t k) {
   return __longlong_as_double((long long)b);
 }
 
-// block-wide sum; every thread gets the result
-__device__ double block_sum(double v, double *red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();
-  if (lane == 0) red[w] = v;
-  __syncthreads();
-  const int nw = blockDim.x >> 5;
-  double t = (lane < nw) ? red[lane] : 0.0;
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  return t;
-}
-
+// block-wide maximum and sum; every thread gets the result
 __device__ double block_max(double v, double *red) {
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -59,8 +47,7 @@ __device__ double block_max(double v, double *red) {
   return t;
 }
 
-// block-wide sum with one barrier: red2 holds two 32-entry buffers used in
-// turn by consecutive calls (a thread may start the next call's write while
+// the sum with one barrier: red2 holds two 32-entry buffers used in turn by consecutive calls (a thread may start the next call's write while
 // others still read this call's buffer, never the same buffer)
 __device__ __forceinline__ double block_sum1(double v, double *red2, int parity) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -86,10 +73,15 @@ __device__ __forceinline__ double block_sum1(double v, double *red2, int parity)
 // last column from row nc - 1 on; M replaces R and the heads of the
 // reflections, V[i + nxb j] for i, j < nc but for its last entry, 1 / D[nc-1].
 // Dynamic shared memory: 2 nc^2 doubles with moments, else none.
+// Latency of one CTA: two passes over a column (L2) and a barrier per pair of
+// columns.  hk_kdist_noalloc, which factorises on each call, on 5 bins, without
+// moments / with f and M formed by reflections of three barriers / so: 10000 x
+// 20 1138 / 1195 / 1083 us, 2858 x 90 7960 / 8760 / 7730, 3000 x 30 1008 / 1046 /
+// 889.
 __global__ void __launch_bounds__(KD_THREADS)
 qr_kernel(int nxb, int nc, int moments, double *__restrict__ V, double *__restrict__ Cv,
           double *__restrict__ D) {
-  __shared__ double red[32];
+  __shared__ double red[64], red_max[32], s_v0, s_head[KD_MAX_NC];
   for (int id = threadIdx.x; id < nxb; id += blockDim.x) {
     const double x = id * 2.0 / ((double)nxb - 1.0) - 1.0;
     V[id] = 1.0;
@@ -103,62 +95,64 @@ qr_kernel(int nxb, int nc, int moments, double *__restrict__ V, double *__restri
     }
   }
   __syncthreads();
+  // Thread tid owns the rows k = tid + n blockDim in every column (nc <= blockDim),
+  // so a sum's barrier is the only one a column needs.
+  const int tid = threadIdx.x, nt = blockDim.x;
+  int par = 0;  // block_sum1's buffer
   for (int i = 0; i < nc; ++i) {
     double *vi = V + (int64_t)nxb * i;
+    const int k0 = tid >= i ? tid : tid + nt;  // the thread's first row at or below i
     double m = 0.0;
-    for (int k = i + threadIdx.x; k < nxb; k += blockDim.x) m = fmax(m, fabs(vi[k]));
-    const double scale = block_max(m, red);
+    for (int k = k0; k < nxb; k += nt) m = fmax(m, fabs(vi[k]));
+    const double scale = block_max(m, red_max);
     double ss = 0.0;
-    for (int k = i + threadIdx.x; k < nxb; k += blockDim.x) {
+    for (int k = k0; k < nxb; k += nt) {
       const double v = vi[k] / scale;
       vi[k] = v;
       ss = __fma_rn(v, v, ss);
     }
-    ss = block_sum(ss, red);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const double s = sqrt(ss);
-      const double v0 = vi[i];
-      const double sigma = (v0 < 0.0) ? -s : s;
+    if (tid == i) s_v0 = vi[i];
+    ss = block_sum1(ss, red, par);  // (its barrier publishes s_v0)
+    par ^= 1;
+    const double s = sqrt(ss), v0 = s_v0;
+    const double sigma = (v0 < 0.0) ? -s : s, c = sigma * (v0 + sigma);
+    if (tid == i) {
       vi[i] = v0 + sigma;
-      Cv[i] = sigma * (v0 + sigma);
+      Cv[i] = c;
       D[i] = -scale * sigma;
     }
-    __syncthreads();
     for (int j = i + 1; j < nc; ++j) {
       double *vj = V + (int64_t)nxb * j;
       double dot = 0.0;
-      for (int k = i + threadIdx.x; k < nxb; k += blockDim.x) dot = __fma_rn(vi[k], vj[k], dot);
-      dot = block_sum(dot, red);
-      const double t = dot / Cv[i];
-      for (int k = i + threadIdx.x; k < nxb; k += blockDim.x) vj[k] = __fma_rn(-t, vi[k], vj[k]);
-      __syncthreads();
+      for (int k = k0; k < nxb; k += nt) dot = __fma_rn(vi[k], vj[k], dot);
+      dot = block_sum1(dot, red, par);
+      par ^= 1;
+      const double t = dot / c;
+      for (int k = k0; k < nxb; k += nt) vj[k] = __fma_rn(-t, vi[k], vj[k]);
     }
   }
   if (!moments) return;
   // f = H_0 (H_1 ( .. H_(nc-2) e_(nc-1))), rows >= nc - 1 in the last column,
-  // the first rows in s_head
-  __shared__ double s_head[KD_MAX_NC];
+  // the first rows in s_head (every thread its own rows, as above)
   double *f = V + (int64_t)nxb * (nc - 1);
-  for (int k = threadIdx.x; k < nxb; k += blockDim.x) {
+  for (int k = tid; k < nxb; k += nt) {
     if (k < nc - 1) s_head[k] = 0.0;
     else f[k] = k == nc - 1 ? 1.0 : 0.0;
   }
-  __syncthreads();
   for (int j = nc - 2; j >= 0; --j) {
     const double *vj = V + (int64_t)nxb * j;
+    const int k0 = tid >= j ? tid : tid + nt;
     double dot = 0.0;
-    for (int k = j + threadIdx.x; k < nxb; k += blockDim.x)
-      dot = __fma_rn(vj[k], k < nc - 1 ? s_head[k] : f[k], dot);
-    dot = block_sum(dot, red);
+    for (int k = k0; k < nxb; k += nt) dot = __fma_rn(vj[k], k < nc - 1 ? s_head[k] : f[k], dot);
+    dot = block_sum1(dot, red, par);
+    par ^= 1;
     const double t = dot / Cv[j];
-    __syncthreads();
-    for (int k = j + threadIdx.x; k < nxb; k += blockDim.x) {
+    for (int k = k0; k < nxb; k += nt) {
       double &w = k < nc - 1 ? s_head[k] : f[k];
       w = __fma_rn(-t, vj[k], w);
     }
-    __syncthreads();
   }
+  __syncthreads();
   // column j of M: the unit vector j through the substitutions, thread j
   extern __shared__ double qr_dyn[];
   double *R = qr_dyn, *X = qr_dyn + nc * nc;  // X[i nc + j]: element i of column j
