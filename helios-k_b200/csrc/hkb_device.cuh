@@ -299,16 +299,34 @@ __device__ __forceinline__ double rcp_d(double v) {
   return __fma_rn(r, e, r);
 }
 
+constexpr int HK_D916_K = 13, HK_D916_MR = 33;
+constexpr double HK_D916_A2 = HK_A916_D * HK_A916_D;
+
+// The table of one line, Y = y^2: f[m-1] = 1 / (a^2 m^2 + Y); returns sig1.
+__device__ __forceinline__ double c916_tab_d(double Y, double *__restrict__ f) {
+  double sig1 = 0.0;
+  double e = exp(-HK_D916_A2), q = exp(-3.0 * HK_D916_A2);  // exp(-a^2 m^2) by its ratios
+  for (int m = 1; m <= HK_D916_MR; ++m) {
+    f[m - 1] = 1.0 / __fma_rn(HK_D916_A2 * m, (double)m, Y);
+    if (m <= HK_D916_K) {
+      sig1 = __fma_rn(e, f[m - 1], sig1);
+      e *= q;
+      q *= 0.606538354524358;  // exp(-2 a^2)
+    }
+  }
+  return sig1;
+}
+
 // Algorithm 916 in FP64 as voigt916_d, for a line whose f[m-1] = 1 / (a^2 m^2 +
 // y^2), m = 1 .. HK_D916_MR, and sig1 = sum_m exp(-a^2 m^2) f[m-1] are at hand
 // (the sum s1 is exp(-x^2) sig1): the Gaussians of s3 run outwards from the
 // term nearest x by their exact ratios exp(-a^2 (2k + 1) -+ 2 a d), d = a mc - |x|,
 // HK_D916_K terms each side (the first omitted one is below 1e-21 of the
 // centre's Gaussian), those of s2 likewise from m = 1: five exponentials per
-// call in place of four per term, and no division.  Against voigt916_d: 9e-16
-// rms, 4e-14 at most (where the formula's terms cancel, |x| < 1, y near 2).
-constexpr int HK_D916_K = 13, HK_D916_MR = 33;
-constexpr double HK_D916_A2 = HK_A916_D * HK_A916_D;
+// call in place of four per term, and no division.  For r < 10 only (f ends at
+// m = 33).  Relative error against 40-digit values: 2.3e-16 rms and 1.8e-15 at
+// most (tiny y, where exp(-x^2) carries x^2 roundings); voigt916_d: 2.6e-16 and
+// 1.8e-15.
 __device__ __forceinline__ double voigt916_tab_d(double x, double y, double ey, double sig1,
                                                  const double *__restrict__ f) {
   const double a = HK_A916_D, a2 = HK_D916_A2;

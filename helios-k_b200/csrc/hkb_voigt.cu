@@ -496,17 +496,7 @@ __device__ __forceinline__ void stage_plain(const LinePrep *__restrict__ P, cons
   r.wide = !(fmax(xa * xa, xb * xb) + Y < 1e300);
   r.sig1 = 0.0;
   if (nonempty && li[3] > li[2]) {
-    // region C in the tile: the denominators and the x-independent sum
-    double e = exp(-HK_D916_A2), q = exp(-3.0 * HK_D916_A2);  // exp(-a^2 m^2) by its ratios
-    for (int m = 1; m <= HK_D916_MR; ++m) {
-      const double f = 1.0 / __fma_rn(HK_D916_A2 * m, (double)m, Y);
-      ftab[m - 1] = f;
-      if (m <= HK_D916_K) {
-        r.sig1 = __fma_rn(e, f, r.sig1);
-        e *= q;
-        q *= 0.606538354524358;  // exp(-2 a^2)
-      }
-    }
+    r.sig1 = c916_tab_d(Y, ftab);  // region C in the tile
   }
   *recp = r;
 }
@@ -1846,7 +1836,12 @@ __global__ void profile_eval_kernel(int64_t n, const double *__restrict__ x,
     out[i] = (double)voigt916_tab((float)x[i], yf, iy, (float)ey, (float)c916_sig1(y[i]),
                                   R + HK_RPAD);
   } else {
-    out[i] = voigt916_d(x[i], y[i], ey);
+    // as the plain Voigt sum: the table that it stages per line, in region C
+    // (its HK_D916_MR terms reach no further)
+    double f[HK_D916_MR];
+    const double Y = y[i] * y[i];
+    if (x[i] * x[i] + Y < 100.0) out[i] = voigt916_tab_d(x[i], y[i], ey, c916_tab_d(Y, f), f);
+    else out[i] = voigt916_d(x[i], y[i], ey);
   }
 }
 
