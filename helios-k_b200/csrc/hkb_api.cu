@@ -930,6 +930,29 @@ hk_status hk_profile_eval(hk_ctx *c, int64_t n, const double *x, const double *y
   return HK_OK;
 }
 
+hk_status hk_fp64_eval(hk_ctx *c, int fn, int64_t n, const double *a, const double *b, double *out) {
+  if (!c || n < 0 || (n > 0 && (!a || !out))) return HK_ERR_ARG;
+  if (fn != 0 && fn != 1) return fail(c, HK_ERR_ARG, "fn must be 0 (reciprocal) or 1 (grid position)");
+  if (n > 0 && fn == 1 && !b) return fail(c, HK_ERR_ARG, "the grid position needs its divisors");
+  for (int64_t i = 0; i < n; ++i)
+    if (fn == 1 && !(a[i] >= 0.0 && a[i] <= b[i] && b[i] >= 1.0 && b[i] <= 2147483647.0 &&
+                     a[i] == std::floor(a[i]) && b[i] == std::floor(b[i])))
+      return fail(c, HK_ERR_ARG, "a grid position needs whole numbers 0 <= j <= den < 2^31, den >= 1");
+  if (n == 0) return HK_OK;
+  cudaSetDevice(c->device);
+  DevBuf w;
+  CUDA_TRY(c, w.ensure(n * 3 * sizeof(double)));
+  double *ad = w.as<double>(), *bd = ad + n, *od = bd + n;
+  cudaError_t e = cudaMemcpy(ad, a, n * 8, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && fn == 1) e = cudaMemcpy(bd, b, n * 8, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = fn == 0 ? launch_rcp(n, ad, od, 0) : launch_grid_pos(n, ad, bd, od, 0);
+  if (e == cudaSuccess) e = cudaMemcpy(out, od, n * 8, cudaMemcpyDeviceToHost);
+  w.release();
+  CUDA_TRY(c, e);
+  ok(c);
+  return HK_OK;
+}
+
 // --------------------------------------------------------------- adjoint
 hk_status hk_set_workspace(hk_ctx *c, double prep_bytes, double part_bytes) {
   if (!c) return HK_ERR_ARG;

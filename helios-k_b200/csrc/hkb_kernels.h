@@ -190,6 +190,12 @@ cudaError_t launch_prep_dump(const LinesDev &L, const GridDev &g,
 cudaError_t launch_profile_eval(int64_t n, const double *x_d, const double *y_d,
                                 int mixed, double *out_d, cudaStream_t stream);
 
+// out = rcp_d(v); out = grid_pos(j, den): the kernels' own reciprocal and grid
+// position
+cudaError_t launch_rcp(int64_t n, const double *v_d, double *out_d, cudaStream_t stream);
+cudaError_t launch_grid_pos(int64_t n, const double *j_d, const double *den_d, double *out_d,
+                            cudaStream_t stream);
+
 size_t kdist_scratch_doubles(int nxb, int nbins, int nstates);
 
 cudaError_t launch_qr(int nxb, int nc, double *V_d, double *C_d, double *D_d,

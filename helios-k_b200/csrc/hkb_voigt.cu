@@ -1845,6 +1845,17 @@ __global__ void profile_eval_kernel(int64_t n, const double *__restrict__ x,
   }
 }
 
+__global__ void rcp_kernel(int64_t n, const double *__restrict__ v, double *__restrict__ out) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = rcp_d(v[i]);
+}
+
+cudaError_t launch_rcp(int64_t n, const double *v_d, double *out_d, cudaStream_t stream) {
+  if (n <= 0) return cudaSuccess;
+  rcp_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(n, v_d, out_d);
+  return cudaGetLastError();
+}
+
 // FP32 FMA throughput probe: 8 independent FMA chains per thread, every SM
 // busy.  Gives the FP32 SIMT peak under the clocks of the current run (the
 // roofline denominator of the Voigt sum).

@@ -68,6 +68,7 @@ def lib():
             "hk_state_lines": (_i, [_p, _d, _d, _p, _p, _p, _p, _p]),
             "hk_line_order": (_i, [_p, _p]),
             "hk_profile_eval": (_i, [_p, _i64, _p, _p, _i, _p]),
+            "hk_fp64_eval": (_i, [_p, _i, _i64, _p, _p, _p]),
             "hk_last_timing": (_i, [_p, _p, _p]),
             "hk_tile_points": (_i, []),
             "hk_fp32_peak": (_i, [_p, _p]),
@@ -462,6 +463,16 @@ class Context:
         y = _f64(y)
         out = np.empty(len(x), np.float64)
         self._chk(lib().hk_profile_eval(self._h, len(x), _ptr(x), _ptr(y), precision, _ptr(out)))
+        return out
+
+    def fp64_eval(self, fn, a, b=None):
+        """The kernels' FP64 helpers: fn 0 the reciprocal of a, 1 the grid position 2 a / b - 1."""
+        a = _f64(a)
+        b = None if b is None else _f64(b)
+        if b is not None and len(b) != len(a):
+            raise ValueError("a and b differ in length")
+        out = np.empty(len(a), np.float64)
+        self._chk(lib().hk_fp64_eval(self._h, fn, len(a), _ptr(a), _ptr(b), _ptr(out)))
         return out
 
     def last_timing(self):

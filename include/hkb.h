@@ -384,6 +384,13 @@ hk_status hk_line_order(hk_ctx *ctx, int64_t *order);
 hk_status hk_profile_eval(hk_ctx *ctx, int64_t n, const double *x,
                           const double *y, int precision, double *out);
 
+/* FP64 helpers of the kernels, evaluated by their device code on host arrays.
+ * fn 0: the reciprocal of a (normal, up to 1e300; b unused) of the plain form's
+ * regions A and B.  fn 1: the grid position 2 a / b - 1 of the Chebyshev fit,
+ * whole numbers 0 <= a <= b < 2^31, b >= 1 (else HK_ERR_ARG). */
+hk_status hk_fp64_eval(hk_ctx *ctx, int fn, int64_t n, const double *a, const double *b,
+                       double *out);
+
 /* Device time of the last hk_opacity / hk_kdist kernels (CUDA events on
  * the launching stream), in milliseconds; and the grid tile size.  After
  * hk_opacity_vjp, voigt_ms is the time of its adjoint kernels. */
