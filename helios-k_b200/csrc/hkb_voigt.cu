@@ -978,23 +978,24 @@ __device__ __forceinline__ void sweep_G(const RecF &r, int wb, int lane,
         inv = rcp_fast(fmaf(x, x, Yf));
       }
       if (EXT == HK_EXT_PL) {
-        float t;
+        float t, w = 1.f;
         if (plc == (inB ? HK_F_PLB : HK_F_PLA)) {
           // (x_c - |x|)(x_c + |x|) = x_c^2 - s; times 1 / (x_c^2 + Y) in
           // region A, times Q(s) / D(x_c^2) in region B
           const float dx = (float)(pe->xd - fabs(fma((double)k, pe->vb, pe->D0)));
-          float w = dx * (pe->xcf + fabsf(x)) * pe->ic;
+          w = dx * (pe->xcf + fabsf(x)) * pe->ic;
           if (inB) w *= fmaf(fmaf(pe->q2, s, pe->q1), s, pe->q0);
-          t = (S1f * inv) * w;
+          t = S1f * inv;
         } else {
           t = fmaf(f, inv, -plf);
         }
+        // (one rounding for t w and its sum, as in sweep_PL)
         if (WEAK) {
-          cacc[k] = fma(S1w, (double)t, cacc[k]);
+          cacc[k] = fma(S1w, (double)(t * w), cacc[k]);
         } else if (p & 1) {
-          a32[p >> 1].y += t;
+          a32[p >> 1].y = fmaf(t, w, a32[p >> 1].y);
         } else {
-          a32[p >> 1].x += t;
+          a32[p >> 1].x = fmaf(t, w, a32[p >> 1].x);
         }
       } else if (EXT == HK_EXT_CHI) {
         float t = f * inv;
@@ -1018,9 +1019,11 @@ __device__ __forceinline__ void sweep_G(const RecF &r, int wb, int lane,
 }
 
 // Plinth removal, a whole slice in one of regions A and B (INB): the terms of
-// sweep_G with its operations in its order (same bits), two points to a packed
-// instruction and no test per point.  FACT: the edge lies in the same region
-// (factored difference), else term - plinth.  kd: the lane's first tile point.
+// sweep_G with its operations in its order (same bits: tests/test_plinth_packed.py),
+// two points to a packed instruction and no test per point.  FACT: the edge lies
+// in the same region (factored difference), else term - plinth.  kd: the lane's
+// first tile point.  (A packed sum of a packed product is written as the FMA
+// that the compiler makes of it, also without contraction: sweep_G has it too.)
 template <bool INB, bool FACT, int PPL>
 __device__ __forceinline__ void sweep_PL(const RecF &rr, const ExtPL &pe, double kd,
                                          const float2 (&kf)[PPL / 2], float2 (&a32)[PPL / 2]) {
@@ -1045,7 +1048,7 @@ __device__ __forceinline__ void sweep_PL(const RecF &rr, const ExtPL &pe, double
                                     (float)(xd - fabs(fma(kd + (64.0 * q + 32.0), vbd, D0))));
       float2 w = __fmul2_rn(__fmul2_rn(dx, __fadd2_rn(xcf, make_float2(fabsf(x.x), fabsf(x.y)))), ic);
       if (INB) w = __fmul2_rn(w, __ffma2_rn(__ffma2_rn(q2, s, q1), s, q0));
-      a32[q] = __fadd2_rn(a32[q], __fmul2_rn(__fmul2_rn(c.S1f, inv), w));
+      a32[q] = __ffma2_rn(__fmul2_rn(c.S1f, inv), w, a32[q]);
     } else {
       a32[q] = __fadd2_rn(a32[q], __ffma2_rn(num, inv, nplf));
     }
@@ -1359,8 +1362,9 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t
             continue;
           }
           if constexpr (EXT == HK_EXT_PL && !G34) {
-            // every class through the generic sweep less the plinth
-            const double u = ldexp(1.0, -(s1exp + HK_LEVEL_BITS * lcur));
+            // whole slices of one region through sweep_PL, every other class
+            // through the generic sweep less the plinth
+            const double u = scale2_d(1.0, -(s1exp + HK_LEVEL_BITS * lcur));
             unsigned mX = m;
             while (mX) {
               const int b = __ffs(mX) - 1;
