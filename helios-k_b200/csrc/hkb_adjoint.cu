@@ -778,6 +778,28 @@ adjoint_line_kernel(LinesDev L, StateDev st, const double *__restrict__ G,
   }
 }
 
+// Parts of a tile's lines, one ticket each.  A ticket stages the tile's u (and
+// its moments) before its first line, so it wants as many lines as its warps can
+// share, at least: 8 of the mixed form, 4 of the plain one, up to 1.5 tickets
+// per resident CTA (tiles at the grid's ends hold fewer lines); more tickets
+// balance better where each still has many lines (150 mixed, 32 plain), up to 8
+// per CTA.  Measured, us by parts of a tile (64 / 100 / 592) and by this rule:
+// mixed, 1 tile x 3e4 lines 313 / 218 / 131, 122; 1 tile x 2000 60 / 55 / 55, 49; 7
+// tiles x 7200 185 / 163 / 214, 164; 19 tiles x 170 89 / 109 / 319, 69; 19 tiles x
+// 17000 814 / 777 / 945, 779; 110 tiles x 55 275 / 367 / 1595, 113; plain (64 / 100 /
+// 296), 8 tiles x 9900 871 / 791 / 686, 684; 25 tiles x 25 74 / 80 / 110, 48.
+// The lines that reach a tile are those spread over the grid and its margins;
+// windows that vary from line to line (cutMode 1, 2) are not known here: there
+// 8 tickets per CTA and at most 64 parts.
+static int adjoint_parts(bool mixed, const GridDev &g, int64_t n, int ntiles, int tpts, int resident) {
+  const int64_t most = (8LL * resident + ntiles - 1) / ntiles;
+  if (g.cutMode != 0) return (int)std::min<int64_t>(64, std::max<int64_t>(1, most));
+  const double reach = 2.0 * g.cut, tile = tpts * g.dnu;
+  const int64_t nL = (int64_t)((double)n * std::min(1.0, (reach + tile) / (reach + (double)g.nx * g.dnu)));
+  const int64_t fill = std::min<int64_t>((3LL * resident / 2 + ntiles - 1) / ntiles, nL / (mixed ? 8 : 4));
+  return (int)std::max<int64_t>(1, std::min(most, std::max(fill, nL / (mixed ? 150 : 32))));
+}
+
 cudaError_t launch_opacity_vjp(bool mixed, const LinesDev &L, const GridDev &g,
                                const StateDev *state_d, const StateDev &state_h,
                                const LinePrep *prep_d, const double *u_d, unsigned *ticket_d,
@@ -801,10 +823,7 @@ cudaError_t launch_opacity_vjp(bool mixed, const LinesDev &L, const GridDev &g,
   else
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, adjoint_tile_kernel, AD_THREADS, 0);
   const int resident = nsm * (per_sm < 1 ? 1 : per_sm);
-  // about 8 tickets per resident CTA, at most 100 parts of a tile's lines (7
-  // tiles of 7200 lines each: 148 us in 64 parts, which leave a quarter of the
-  // resident CTAs without a ticket, 127 us in 100, 134 us in 170)
-  const int nsplit = (int)std::min<int64_t>(100, std::max<int64_t>(1, (8LL * resident + ntiles - 1) / ntiles));
+  const int nsplit = adjoint_parts(mixed, g, L.n, ntiles, tpts, resident);
   const int ctas = (int)std::min<int64_t>((int64_t)ntiles * nsplit, resident);
   if (mixed) {
     adjoint_ab_kernel<<<ctas, AD_THREADS, 0, stream>>>(prep_d, L.nu0, L.n, g, state_d, ntiles, nsplit,
