@@ -1058,15 +1058,18 @@ __device__ __forceinline__ void sweep_PL(const RecF &rr, const ExtPL &pe, double
 // Plinth removal, a line summed per point in FP64 (HK_F_PL64: its cut edge
 // lies in region C or close to a region boundary, or FP32 cannot hold it):
 // the FP64 form's terms (regions C, B, A) less the plinth, from the line's
-// FP64 vy, erfcx(vy) and plinth (pe) and x = D0 + k vb.
+// FP64 vy, erfcx(vy) and plinth (pe) and x = D0 + k vb.  Out of line, four points
+// at a time: inline, it shared the packed sweeps' registers, and states made of
+// such lines ran up to 5 % slower than before those (7389 lines x 44760 points at
+// 5.4 atm 384 -> 401 us, 382 so; 13488 x 125150 at 0.07 atm 734 -> 747, 680 so).
 template <int PPL>
-__device__ __forceinline__ void sweep_pl64(const RecF &r, const ExtPL &pe, int wb, int lane,
+__device__ __noinline__ void sweep_pl64(const RecF &r, const ExtPL &pe, int wb, int lane,
                                            double *__restrict__ cacc, int profile) {
   const int we = wb + 32 * PPL;
   if (r.i1 <= wb || r.i0 >= we) return;
   const double vy = pe.vy, Y = vy * vy;
   const double S1 = r.Sc * vy * 0.56418958354775628;  // S vy / pi
-#pragma unroll 1
+#pragma unroll 4
   for (int p = 0; p < PPL; ++p) {
     const int k = wb + lane + 32 * p;
     if (k >= r.i0 && k < r.i1) {
