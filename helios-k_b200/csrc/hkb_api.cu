@@ -1208,11 +1208,12 @@ hk_status hk_opacity_vjp_log(hk_ctx *c, double T, double P, int precision, const
 // Two ways to record a table, with the same bits: the per-batch launches
 // (line prep, scale, Voigt sum per batch of states whose records fit the
 // workspace; the default, the faster one measured on the 1e7-line, 600-state
-// table: 28.6 ms per state against 30.1) and, with hk_set_table_mode(ctx, 1),
+// table: 21.4 ms per state against 24.2) and, with hk_set_table_mode(ctx, 1),
 // one persistent launch for every state's line prep and sums (two kernels in
 // the graph).  Tables of fewer states than this always take the per-batch
 // launches: the fused launch can only hide a state's line prep behind
-// another state's sums (one 1e7-line state: 31.1 ms per-batch, 32.8 fused).
+// another state's sums (one 1e7-line state, both before the far field: 31.1 ms
+// per-batch, 32.8 fused).
 constexpr int HK_TABLE_FUSED_MIN = 4;
 
 hk_status hk_set_table_mode(hk_ctx *c, int fused) {
