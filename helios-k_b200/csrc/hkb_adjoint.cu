@@ -782,12 +782,13 @@ adjoint_line_kernel(LinesDev L, StateDev st, const double *__restrict__ G,
 // its moments) before its first line, so it wants as many lines as its warps can
 // share, at least: 8 of the mixed form, 4 of the plain one, up to 1.5 tickets
 // per resident CTA (tiles at the grid's ends hold fewer lines); more tickets
-// balance better where each still has many lines (150 mixed, 32 plain), up to 8
+// balance better where each still has many lines (150 mixed, 16 plain), up to 8
 // per CTA.  Measured, us by parts of a tile (64 / 100 / 592) and by this rule:
 // mixed, 1 tile x 3e4 lines 313 / 218 / 131, 122; 1 tile x 2000 60 / 55 / 55, 49; 7
 // tiles x 7200 185 / 163 / 214, 164; 19 tiles x 170 89 / 109 / 319, 69; 19 tiles x
 // 17000 814 / 777 / 945, 779; 110 tiles x 55 275 / 367 / 1595, 113; plain (64 / 100 /
-// 296), 8 tiles x 9900 871 / 791 / 686, 684; 25 tiles x 25 74 / 80 / 110, 48.
+// 150), 8 tiles x 6600 585 / 547 / 492, 449; 40 tiles x 415 201 / 255 / 347, 214; 25
+// tiles x 25 73 / 79 / 87, 48.
 // The lines that reach a tile are those spread over the grid and its margins;
 // windows that vary from line to line (cutMode 1, 2) are not known here: there
 // 8 tickets per CTA and at most 64 parts.
@@ -797,7 +798,7 @@ static int adjoint_parts(bool mixed, const GridDev &g, int64_t n, int ntiles, in
   const double reach = 2.0 * g.cut, tile = tpts * g.dnu;
   const int64_t nL = (int64_t)((double)n * std::min(1.0, (reach + tile) / (reach + (double)g.nx * g.dnu)));
   const int64_t fill = std::min<int64_t>((3LL * resident / 2 + ntiles - 1) / ntiles, nL / (mixed ? 8 : 4));
-  return (int)std::max<int64_t>(1, std::min(most, std::max(fill, nL / (mixed ? 150 : 32))));
+  return (int)std::max<int64_t>(1, std::min(most, std::max(fill, nL / (mixed ? 150 : 16))));
 }
 
 cudaError_t launch_opacity_vjp(bool mixed, const LinesDev &L, const GridDev &g,
