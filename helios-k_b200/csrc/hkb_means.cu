@@ -135,13 +135,21 @@ constexpr int TR_SMEM_MAX = 200 * 1024;  // values that do not fit stay in globa
 // sums sum_k ((K_k - c) / h)^p / p! formed once per bin.
 constexpr int TR_B = 32, TR_P = 18;
 
+// Bins below this many points, or this many exponentials, are summed value by
+// value: forming the power sums takes each block's thread a few us (300 bins,
+// with / without them: 300 points and 10 m_j 58 / 42 us, 1000 m_j 572 / 598; 1000
+// points and 10 m_j 67 / 54, 100 m_j 132 / 147, 1000 m_j 631 / 997).
+constexpr int TR_MIN_NXB = 512, TR_MIN_EXPS = 30000;
+
 // doubles of shared memory per block: c, h, the smallest value, TR_P + 1 sums
 constexpr int TR_W = TR_P + 4;
 static size_t tr_words(int nxb) { return (size_t)((nxb + TR_B - 1) / TR_B) * TR_W * sizeof(double); }
 
 // 180 bins of 10000 values x 1000 m_j: 4.58 ms with an exponential per value
 // (1.8e9 of them), 0.59 ms so (about 40 of 313 blocks per m_j still value by
-// value).  Bound: instruction issue (77 % of slots; FP64 pipe 43 %).
+// value).  Bound: instruction issue (77 % of slots; FP64 pipe 43 %).  Unsorted
+// values of 13 decades, whose blocks are all too wide: 300 bins of 10000 x 100 m_j
+// 824 us value by value, 1098 with power sums that no m_j can use, 813 without.
 __global__ void __launch_bounds__(TR_THREADS)
 transmission_kernel(const double *__restrict__ K, int64_t k_stride, int nxb, int nbins,
                     const int *__restrict__ nxmin, double kmin, int nTr, double dTr, int use_smem,
@@ -160,6 +168,8 @@ transmission_kernel(const double *__restrict__ K, int64_t k_stride, int nxb, int
     kb = kb_s;
   }
   if (poly_ok) {
+    // the third smallest m_j
+    const double m3 = exp(fmin(-(nTr / 2) * dTr, (nTr - 1 - nTr / 2) * dTr) + 2.0 * fabs(dTr));
     for (int q = threadIdx.x; q < nblk; q += TR_THREADS) {
       // (each lane starts at another value of its block: no bank conflicts)
       const int k0 = q * TR_B, nk = min(TR_B, nxb - k0);
@@ -174,12 +184,14 @@ transmission_kernel(const double *__restrict__ K, int64_t k_stride, int nxb, int
         finite = finite && isfinite(v);
       }
       const double c = 0.5 * lo + 0.5 * hi, h = 0.5 * hi - 0.5 * lo, ih = h > 0.0 ? 1.0 / h : 0.0;
-      // (a spread too small to divide by, or a value that is not finite: value by value)
-      const bool ok = finite && (h == 0.0 || isfinite(ih));
+      // (a spread too small to divide by, or a value that is not finite: value by
+      // value; so a spread too wide for all but the two smallest m_j, whose power
+      // sums would cost more than they save)
+      const bool ok = finite && (h == 0.0 || isfinite(ih)) && h * m3 <= 1.0;
       double a[TR_P + 1];
 #pragma unroll
       for (int p = 0; p <= TR_P; ++p) a[p] = 0.0;
-      for (int i = 0; i < TR_B; ++i) {
+      for (int i = 0; i < TR_B && ok; ++i) {
         const int k = (i + lane) & (TR_B - 1);
         if (k >= nk) continue;
         const double t = (kb[k0 + k] - c) * ih;
@@ -222,7 +234,15 @@ transmission_kernel(const double *__restrict__ K, int64_t k_stride, int nxb, int
           for (int p = TR_P - 1; p >= 0; --p) t = __fma_rn(t, d, w[(3 + p) * nblk + q]);
           a = __fma_rn(exp(-w[q] * m), t, a);
         }
-        for (unsigned e = __ballot_sync(0xffffffffu, each); e; e &= e - 1) {
+        unsigned e = __ballot_sync(0xffffffffu, each);
+        if (e == __ballot_sync(0xffffffffu, q < nblk)) {
+          // every block of the group (unsorted values): one loop over them
+          const int end = min(nxb, (q0 + 32) * TR_B);
+#pragma unroll 4
+          for (int k = q0 * TR_B + lane; k < end; k += 32) a += exp(-kb[k] * m);
+          e = 0u;
+        }
+        for (; e; e &= e - 1) {
           const int k = (q0 + __ffs(e) - 1) * TR_B + lane;
           if (k < nxb) a += exp(-kb[k] * m);
         }
@@ -249,7 +269,7 @@ cudaError_t launch_transmission(const double *K_d, int64_t k_stride, int nstates
                                 double *Tr_d, cudaStream_t stream) {
   if (nstates <= 0 || nbins <= 0 || nTr <= 0) return cudaSuccess;
   const size_t words = tr_words(nxb), vals = (size_t)nxb * sizeof(double);
-  const int poly_ok = words <= (size_t)TR_SMEM_MAX;
+  const int poly_ok = words <= (size_t)TR_SMEM_MAX && nxb >= TR_MIN_NXB && (int64_t)nxb * nTr >= TR_MIN_EXPS;
   const int use_smem = vals + (poly_ok ? words : 0) <= (size_t)TR_SMEM_MAX;
   const size_t smem = (use_smem ? vals : 0) + (poly_ok ? words : 0);
   if (smem > 48 * 1024) {
