@@ -126,9 +126,10 @@ constexpr int HK_F_WEAK = 1, HK_F_WIDE = 2, HK_F_PLA = 4, HK_F_PLB = 8, HK_F_PL6
 constexpr int HK_LEVEL_BITS = 96;
 constexpr int HK_MAX_LEVEL = 7;
 
-// Options of the mixed form with their own kernel instantiations: none,
-// sub-Lorentzian wings (chi factor), plinth removal.
-enum { HK_EXT_NONE = 0, HK_EXT_CHI = 1, HK_EXT_PL = 2 };
+// Options with their own kernel instantiations: none; in the mixed form,
+// sub-Lorentzian wings (chi factor) and plinth removal; in the plain form, any
+// of profiles 2-4, sub-Lorentzian wings and plinth removal.
+enum { HK_EXT_NONE = 0, HK_EXT_CHI = 1, HK_EXT_PL = 2, HK_EXT_OPT = 3 };
 
 // Per staged line with plinth removal (shared memory, beside its RecF):
 // x = D0 + k vb in FP64 (k the tile-local point), and
@@ -168,11 +169,12 @@ struct __align__(16) RecD {
   int i0, b0, c0, c1, b1, i1, wide, p1;   // wide: x^2 + y^2 may pass 1e300
 };
 
-// Shared memory of one plain CTA: staged records, the per-line region-C tables
-// and the tile's region-C sums.
-template <class SH, int SUB = 1>
+// Shared memory of one plain CTA: staged records and, without options, the
+// per-line region-C tables and the tile's region-C sums.
+template <class SH, int SUB = 1, int EXT = HK_EXT_NONE>
 constexpr size_t smem_plain() {
-  return sizeof(RecD) * SH::CH + sizeof(double) * SH::CH * HK_D916_MR + sizeof(double) * (SH::G / SUB);
+  return sizeof(RecD) * SH::CH +
+         (EXT == HK_EXT_NONE ? sizeof(double) * SH::CH * HK_D916_MR + sizeof(double) * (SH::G / SUB) : 0);
 }
 
 // first index in [0, n) with a[idx] >= v (n if none); all 32 lanes call it
@@ -461,7 +463,7 @@ __device__ __forceinline__ void stage_rtab(float y, float *__restrict__ Rtab) {
   for (int m = 1; m <= HK_C916_MR; ++m) Rtab[m - 1] = rcp_fast(fmaf(a2 * m, (float)m, Yf));
 }
 
-template <bool CG>
+template <bool CG, int EXT>
 __device__ __forceinline__ void stage_plain(const LinePrep *__restrict__ P, const GridDev &g, int64_t l,
                                             int64_t g0, int64_t g1, RecD *recp, double *ftab) {
   const LinePrep lp = load_record<CG>(P + l);
@@ -485,18 +487,18 @@ __device__ __forceinline__ void stage_plain(const LinePrep *__restrict__ P, cons
   r.b1 = li[4];
   r.i1 = nonempty ? li[5] : 0;
   r.p1 = 0;
-  const double Y = r.y2;
-  const double A2 = 2.0 * Y + (3.0 - 6.0 / CUDART_PI), B2 = (Y + 1.5) * (Y + 1.5);
-  r.C1 = lp.S1 * (2.0 * Y + (2.5 - 4.0 / CUDART_PI));
-  r.C0 = lp.S1 * ((Y + 1.5) * (Y + 1.0));
-  r.D2 = A2 + Y;
-  r.D1 = __fma_rn(A2, Y, B2);
-  r.D0 = B2 * Y;
-  const double xa = (grid_x(g, g0) - lp.nu) * lp.iad, xb = (grid_x(g, g1 - 1) - lp.nu) * lp.iad;
-  r.wide = !(fmax(xa * xa, xb * xb) + Y < 1e300);
-  r.sig1 = 0.0;
-  if (nonempty && li[3] > li[2]) {
-    r.sig1 = c916_tab_d(Y, ftab);  // region C in the tile
+  if (EXT == HK_EXT_NONE) {  // (sweep_plain_opt reads none of these)
+    const double Y = r.y2;
+    const double A2 = 2.0 * Y + (3.0 - 6.0 / CUDART_PI), B2 = (Y + 1.5) * (Y + 1.5);
+    r.C1 = lp.S1 * (2.0 * Y + (2.5 - 4.0 / CUDART_PI));
+    r.C0 = lp.S1 * ((Y + 1.5) * (Y + 1.0));
+    r.D2 = A2 + Y;
+    r.D1 = __fma_rn(A2, Y, B2);
+    r.D0 = B2 * Y;
+    const double xa = (grid_x(g, g0) - lp.nu) * lp.iad, xb = (grid_x(g, g1 - 1) - lp.nu) * lp.iad;
+    r.wide = !(fmax(xa * xa, xb * xb) + Y < 1e300);
+    r.sig1 = 0.0;
+    if (nonempty && li[3] > li[2]) r.sig1 = c916_tab_d(Y, ftab);  // region C in the tile
   }
   *recp = r;
 }
@@ -1084,6 +1086,38 @@ __device__ __noinline__ void sweep_pl64(const RecF &r, const ExtPL &pe, int wb, 
 }
 
 // ------------------------------------------------------------ FP64 sweep
+// Profiles 2-4 (region A only), sub-Lorentzian wings and plinth removal:
+// Line6fA/B/C(X) add the profile (times chi x/nu), then subtract the line's
+// plinth, at every window point.  Its own kernels, and the line's values in
+// registers before its points: 1e5 lines x 3e5 points, Lorentz / Voigt with plinth
+// removal / with sub-Lorentzian wings, us: 2616 / 3451 / 5363 in a kernel that also
+// had the quotient sweep of one division per pair, 3143 / 3857 / 5950 beside the
+// sweep below, 2106 / 3308 / 4916 so.
+template <int PPL>
+__device__ __forceinline__ void sweep_plain_opt(const RecD &r, int wb, int lane,
+                                                const double (&xg)[PPL],
+                                                double (&acc)[PPL], const GridDev &g,
+                                                const StateDev &st) {
+  const int we = wb + 32 * PPL;
+  if (r.i1 <= wb || r.i0 >= we) return;
+  const double nu = r.nu, iad = r.iad, vb = g.dnu * iad;
+  const int i0 = r.i0, i1 = r.i1, b0 = r.b0, b1 = r.b1, c0 = r.c0, c1 = r.c1;
+#pragma unroll
+  for (int p = 0; p < PPL; ++p) {
+    const int k = wb + lane + 32 * p;
+    if (k >= i0 && k < i1) {
+      const double x = (xg[p] - nu) * iad;
+      double v;
+      if (k >= c0 && k < c1) v = r.Sc * voigt916_d(x, r.y, r.ey);
+      else if (k >= b0 && k < b1) v = r.S1 * gh2_d(x, r.y2);
+      else v = profile_a_d(g.profile, x, r.y2, r.S1, vb);
+      if (g.subL) v *= sublorentz_d(g, st, xg[p], nu);
+      acc[p] += v;
+      acc[p] -= r.pl;
+    }
+  }
+}
+
 // One FP64 division per pair and, in region C, four exponentials and three
 // divisions per term of the series bounded it: now a region-B pair is 13 FP64
 // operations (GH2 as one quotient of polynomials with every coefficient
@@ -1094,33 +1128,11 @@ __device__ __noinline__ void sweep_pl64(const RecF &r, const ExtPL &pe, int wb, 
 template <int PPL>
 __device__ __forceinline__ void sweep_plain(const RecD &r, int wb, int lane,
                                             const double (&xg)[PPL],
-                                            double (&acc)[PPL], const GridDev &g,
-                                            const StateDev &st, int64_t g0,
+                                            double (&acc)[PPL], const GridDev &g, int64_t g0,
                                             const double *__restrict__ ftab,
                                             double *__restrict__ cacc) {
   const int we = wb + 32 * PPL;
   if (r.i1 <= wb || r.i0 >= we) return;
-  if (g.profile != 1 || g.plinth || g.subL) {
-    // profiles 2-4 (region A only), sub-Lorentzian wings and plinth removal:
-    // Line6fA/B/C(X) add the profile (times chi x/nu), then subtract the
-    // line's plinth, at every window point
-    const double vb = g.dnu * r.iad;
-#pragma unroll
-    for (int p = 0; p < PPL; ++p) {
-      const int k = wb + lane + 32 * p;
-      if (k >= r.i0 && k < r.i1) {
-        const double x = (xg[p] - r.nu) * r.iad;
-        double v;
-        if (k >= r.c0 && k < r.c1) v = r.Sc * voigt916_d(x, r.y, r.ey);
-        else if (k >= r.b0 && k < r.b1) v = r.S1 * gh2_d(x, r.y2);
-        else v = profile_a_d(g.profile, x, r.y2, r.S1, vb);
-        if (g.subL) v *= sublorentz_d(g, st, xg[p], r.nu);
-        acc[p] += v;
-        acc[p] -= r.pl;
-      }
-    }
-    return;
-  }
   const double S1 = r.S1, Y = r.y2, nu = r.nu, iad = r.iad;
   const bool full = r.i0 <= wb && r.i1 >= we;
   if (full && !r.wide && ((r.b0 <= wb && r.c0 >= we) || (r.c1 <= wb && r.b1 >= we))) {
@@ -1218,7 +1230,8 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t
   using Rec = typename std::conditional<MIXED, RecF, RecD>::type;
   constexpr int CH = SH::CH, PPL = SH::PPL / SUB, SLICE = SH::SLICE, G = SH::G;
   constexpr int SL = SLICE / SUB, GS = G / SUB;  // points per warp and CTA
-  static_assert(SUB == 1 || (SL % HK_FB == 0 && PPL % 2 == 0 && EXT == HK_EXT_NONE && !G34), "sub-tiles");
+  constexpr bool OPT = !MIXED && EXT != HK_EXT_NONE;  // the plain form's options: no shared sums
+  static_assert(SUB == 1 || (SL % HK_FB == 0 && PPL % 2 == 0 && (OPT || EXT == HK_EXT_NONE) && !G34), "sub-tiles");
   // the far field runs in the mixed form without options (Voigt, Lorentz)
   constexpr bool FAR = MIXED && !G34 && EXT == HK_EXT_NONE;
   constexpr int NBLK = GS / HK_FB;  // 64-point blocks of the CTA's points
@@ -1271,7 +1284,7 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t
     } else {
       xg[p] = grid_x(g, g0 + k);
     }
-    cacc[k] = 0.0;  // owned by this warp only: no barrier needed
+    if (!OPT) cacc[k] = 0.0;  // owned by this warp only: no barrier needed
   }
 
   // Chunk c holds the lines L0 + c + q*nch (q < CH): every chunk spans
@@ -1321,7 +1334,7 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t
         if (r.c1 > r.c0 && r.i1 > r.i0) stage_rtab(r.y, Rtab + pos * HK_C916_MR);
       }
     } else if (tid < cnt_c) {
-      stage_plain<CG>(P, g, L0 + c + (int64_t)tid * nch, g0, g1, reinterpret_cast<RecD *>(rec) + tid,
+      stage_plain<CG, EXT>(P, g, L0 + c + (int64_t)tid * nch, g0, g1, reinterpret_cast<RecD *>(rec) + tid,
                       ftab + tid * HK_D916_MR);
     }
     __syncthreads();
@@ -1498,9 +1511,11 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t
         }
       }
     } else {
-      for (int j = 0; j < cnt_c; ++j)
-        sweep_plain<PPL>(reinterpret_cast<const RecD &>(rec[j]), wb, lane, xg, acc, g, st, g0,
-                         ftab + j * HK_D916_MR, cacc);
+      for (int j = 0; j < cnt_c; ++j) {
+        const RecD &r = reinterpret_cast<const RecD &>(rec[j]);
+        if constexpr (OPT) sweep_plain_opt<PPL>(r, wb, lane, xg, acc, g, st);
+        else sweep_plain<PPL>(r, wb, lane, xg, acc, g, g0, ftab + j * HK_D916_MR, cacc);
+      }
     }
     __syncthreads();
   }
@@ -1531,7 +1546,7 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t
     for (int p = 0; p < PPL; ++p) {
       const int k = wb + lane + 32 * p;
       const int64_t gi = g0 + k;
-      acc[p] = MIXED ? cacc[k] : acc[p] + cacc[k];
+      if (!OPT) acc[p] = MIXED ? cacc[k] : acc[p] + cacc[k];
       if (gi < g1) Ks[gi] = st.kmin + acc[p];
     }
   } else {
@@ -1542,7 +1557,7 @@ __device__ __forceinline__ void sum_tile(const void *prep_s, int64_t L0, int64_t
 #pragma unroll
     for (int p = 0; p < PPL; ++p) {
       const int k = wb + lane + 32 * p;
-      acc[p] = MIXED ? cacc[k] : acc[p] + cacc[k];
+      if (!OPT) acc[p] = MIXED ? cacc[k] : acc[p] + cacc[k];
       pt[(int64_t)part * G + k] = acc[p];
     }
     __threadfence();
@@ -1913,10 +1928,11 @@ int voigt_tile_points(int shape) { return HK_SHAPE_G[shape < 0 || shape >= HK_NS
 int voigt_chunk_lines(int shape) { return HK_SHAPE_CH[shape < 0 || shape >= HK_NSHAPES ? 0 : shape]; }
 int voigt_tile_warps(int shape) { return HK_SHAPE_WARPS[shape < 0 || shape >= HK_NSHAPES ? 0 : shape]; }
 
-// The option instantiation of the mixed form for a grid's options (the
-// host runs sub-Lorentzian wings with plinth removal, and the Gaussian
-// profiles with sub-Lorentzian wings, in the FP64 form).
-static int ext_kind(const GridDev &g) {
+// The instantiation for a grid's options (the host runs sub-Lorentzian wings
+// with plinth removal, and the Gaussian profiles with sub-Lorentzian wings, in
+// the FP64 form).
+static int ext_kind(bool mixed, const GridDev &g) {
+  if (!mixed) return g.profile != 1 || g.subL || g.plinth ? HK_EXT_OPT : HK_EXT_NONE;
   if (g.subL) return HK_EXT_CHI;
   if (g.plinth) return HK_EXT_PL;
   return HK_EXT_NONE;
@@ -1936,14 +1952,19 @@ static cudaError_t with_kernel(bool mixed, int shape, F &&f, bool g34 = false, i
   case n:                                                                                             \
     return mixed ? f((KFn)voigt_sum_kernel<true, Shape0, false, HK_EXT_NONE, n>,                      \
                      smem_mixed<Shape0, HK_EXT_NONE, n>(), Shape0::THREADS)                           \
-                 : f((KFn)voigt_sum_kernel<false, Shape0, false, HK_EXT_NONE, n>,                     \
-                     smem_plain<Shape0, n>(), Shape0::THREADS);
+           : ext == HK_EXT_OPT ? f((KFn)voigt_sum_kernel<false, Shape0, false, HK_EXT_OPT, n>,        \
+                                   smem_plain<Shape0, n, HK_EXT_OPT>(), Shape0::THREADS)              \
+                               : f((KFn)voigt_sum_kernel<false, Shape0, false, HK_EXT_NONE, n>,       \
+                                   smem_plain<Shape0, n>(), Shape0::THREADS);
   switch (sub) {
     HK_SUB_CASE(2)
     HK_SUB_CASE(HK_MAX_SUB)
     default: break;
   }
 #undef HK_SUB_CASE
+  if (ext == HK_EXT_OPT)
+    return f((KFn)voigt_sum_kernel<false, Shape0, false, HK_EXT_OPT>, smem_plain<Shape0, 1, HK_EXT_OPT>(),
+             Shape0::THREADS);
   if (!mixed) return f((KFn)voigt_sum_kernel<false, Shape0>, smem_plain<Shape0>(), Shape0::THREADS);
   if (g34 && ext == HK_EXT_PL)
     return f((KFn)voigt_sum_kernel<true, Shape0, true, HK_EXT_PL>, smem_mixed<Shape0, HK_EXT_PL>(),
@@ -2060,8 +2081,8 @@ cudaError_t launch_voigt_sum(bool mixed, const VoigtPlan &pl, const void *prep_d
   if (mixed && (g.profile >= 3 || g.plinth || g.subL) && pl.shape != 0)
     return cudaErrorInvalidValue;  // shape 0 only
   const bool g34 = mixed && g.profile >= 3;
-  const int ext = mixed ? ext_kind(g) : HK_EXT_NONE;
-  const int sub = (pl.shape == 0 && !g34 && ext == HK_EXT_NONE) ? sub_tiles(mixed, pl, nlines, g) : 1;
+  const int ext = ext_kind(mixed, g);
+  const int sub = (pl.shape == 0 && !g34 && (!mixed || ext == HK_EXT_NONE)) ? sub_tiles(mixed, pl, nlines, g) : 1;
   const int total = (int)total64 * sub;
   if (total <= 0) return cudaSuccess;
   if (!work_d || (pl.nsplit > 1 && !partial_d)) return cudaErrorInvalidValue;
@@ -2092,6 +2113,9 @@ static cudaError_t with_table_kernel(bool mixed, int shape, F &&f, bool g34 = fa
   using KFn = void (*)(LinesDev, GridDev, const StateDev *, TableSched, void *, double *, unsigned *,
                        unsigned long long *, unsigned long long *, unsigned *, unsigned *, unsigned *,
                        TableFin *, int *, double *, int64_t);
+  if (ext == HK_EXT_OPT)
+    return f((KFn)voigt_table_kernel<false, Shape0, false, HK_EXT_OPT>, smem_plain<Shape0, 1, HK_EXT_OPT>(),
+             Shape0::THREADS);
   if (!mixed) return f((KFn)voigt_table_kernel<false, Shape0>, smem_plain<Shape0>(), Shape0::THREADS);
   if (g34 && ext == HK_EXT_PL)
     return f((KFn)voigt_table_kernel<true, Shape0, true, HK_EXT_PL>, smem_mixed<Shape0, HK_EXT_PL>(),
@@ -2188,7 +2212,7 @@ cudaError_t launch_voigt_table(bool mixed, const TablePlan &tp, const LinesDev &
     kfn<<<ctas, threads, smem, stream>>>(L, g, states_d, sc, b.ring, b.partial, b.tile_cnt, ticket, wbits,
                                          prep_cnt, sum_cnt, ready, fin, err, K_d, k_stride);
     return cudaGetLastError();
-  }, mixed && g.profile >= 3, mixed ? ext_kind(g) : HK_EXT_NONE);
+  }, mixed && g.profile >= 3, ext_kind(mixed, g));
 }
 
 int *table_error_word(void *sync_d, int nstates) {
