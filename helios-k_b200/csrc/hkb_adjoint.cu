@@ -591,7 +591,7 @@ adjoint_ab_kernel(const LinePrep *__restrict__ P, const double *__restrict__ nu0
 // line's sums to G only where its share enters another line.  (One pair per
 // lane in order ran both evaluators in most steps and closed each step with a
 // segmented scan of four FP64 sums: 1e6 lines with about 28 points each 1.14
-// ms, so 0.70 ms; latency at 118 registers, 16 warps per SM, the smaller
+// ms, so 0.70 ms; latency at 116 registers, 16 warps per SM, the smaller
 // budgets spill.)
 constexpr int AC_WARPS = AD_THREADS / 32;
 struct __align__(16) AcLine {

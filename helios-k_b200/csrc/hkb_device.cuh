@@ -293,8 +293,8 @@ static __device__ __noinline__ double voigt916_d(double x, double y, double ey) 
 // with e = 1 - v r, from the PTX instruction rcp.approx.ftz.f64.  The step
 // leaves e^3 (2^-57), so its result carries the one rounding of the last FMA:
 // relative error at most 1.00 x 2^-53 over all exponents and 507 mantissas each,
-// as a division's (tests/test_fp64_helpers.py).  6e4 lines x 3e5 points: 622 us,
-// 799 with a division in its place.
+// as a division's (tests/test_fp64_helpers.py).  6e4 lines x 3e5 points: 570 us,
+// 753 with a division in its place.
 __device__ __forceinline__ double rcp_d(double v) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(v));

@@ -112,7 +112,7 @@ cudaError_t sort_lines_by_nu(int64_t n, double *nu_d, int64_t *order_d,
 // per state: {half-width bits, term bits} (both non-negative doubles, so
 // their bit patterns order like the values).
 // Threads per CTA of the line prep, 4 CTAs per SM: ~1500 instructions per line
-// (a third FP64), about 100 registers.  1e7 lines of one state: 1.15 ms with the
+// (a third FP64), 128 registers.  1e7 lines of one state: 1.15 ms with the
 // window searches out of line, 0.76 ms with their estimates tried inline (20
 // warps per SM at 96 registers spill: 0.81 ms); 1.12 GB of records and 0.4 GB
 // of columns would take 0.23 ms.  Bound: issue and FP64 latency at 16 warps.

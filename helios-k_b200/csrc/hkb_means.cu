@@ -146,8 +146,8 @@ constexpr int TR_W = TR_P + 4;
 static size_t tr_words(int nxb) { return (size_t)((nxb + TR_B - 1) / TR_B) * TR_W * sizeof(double); }
 
 // 180 bins of 10000 values x 1000 m_j: 4.58 ms with an exponential per value
-// (1.8e9 of them), 0.59 ms so (about 40 of 313 blocks per m_j still value by
-// value).  Bound: instruction issue (77 % of slots; FP64 pipe 43 %).  Unsorted
+// (1.8e9 of them), 0.58 ms so (about 40 of 313 blocks per m_j still value by
+// value).  Bound: instruction issue (74 % of slots; FP64 pipe 43 %).  Unsorted
 // values of 13 decades, whose blocks are all too wide: 300 bins of 10000 x 100 m_j
 // 824 us value by value, 1098 with power sums that no m_j can use, 813 without.
 __global__ void __launch_bounds__(TR_THREADS)

@@ -223,10 +223,11 @@ __device__ __forceinline__ float2 f2(double v) {
 // summed in FP64 (weak), HK_MAX_LEVEL + 2 for lines without points in the
 // tile -- and stage_mixed builds the record for that key.
 // v 2^e as ldexp gives it, |e| <= 2000.  A product of three: ldexp's code and
-// branches sat in the level flushes and in the staging, and this kernel pays
-// for code size (64 registers, several thousand instructions, "no instruction"
-// stalls): 24-state table 14.67 -> 13.56 ms, 4 ExoMol states 19.18 -> 18.63, 1e5
-// lines x 3e6 points with the fit 724 -> 683 us.
+// branches sat in the level flushes and in the staging of a kernel of several
+// thousand instructions at 64 registers ("no instruction" 0.93 -> 0.56 warps per
+// issue with the sort key's and the far flush's code that went with it, issue
+// slots 78 -> 81 %): 24-state table 14.67 -> 13.56 ms, 4 ExoMol states 19.18 ->
+// 18.63, 1e5 lines x 3e6 points with the fit 724 -> 683 us.
 __device__ __forceinline__ double scale2_d(double v, int e) {
   const int h = e >> 1;
   return v * __hiloint2double((1023 + h) << 20, 0) * __hiloint2double((1023 + e - h) << 20, 0);
@@ -1123,8 +1124,9 @@ __device__ __forceinline__ void sweep_plain_opt(const RecD &r, int wb, int lane,
 // operations (GH2 as one quotient of polynomials with every coefficient
 // positive, rcp_d) and region C, its points packed over the lanes, takes its
 // denominators from a table per staged line (voigt916_tab_d).  6e4 lines x 3e5
-// points: 1216 -> 625 us.  Now latency: 16 warps per SM at 128 registers (80
-// registers for 24 warps spill: 695 us), FP64 pipe 32 %.
+// points: 1216 -> 622 us, 569 without the option forms in the kernel.  Now latency:
+// 16 warps per SM at 128 registers (80 registers for 24 warps spill: 695 us against
+// 622), FP64 pipe 35 %.
 template <int PPL>
 __device__ __forceinline__ void sweep_plain(const RecD &r, int wb, int lane,
                                             const double (&xg)[PPL],
@@ -1194,8 +1196,7 @@ __device__ __forceinline__ void flush_sums(float2 (&a32)[PPL / 2], double *__res
 
 // The nu-sorted lines whose windows can reach grid points [g0, g1), wmax the
 // state's search half-width and shift its largest pressure shift: the first
-// (end = false) or past the last; all 32
-// lanes call it.
+// (end = false) or past the last; all 32 lanes call it.
 __device__ __forceinline__ int64_t tile_lines(const double *__restrict__ nu0, int64_t nlines,
                                               const GridDev &g, double shift, double wmax,
                                               int64_t g0, int64_t g1, bool end) {
