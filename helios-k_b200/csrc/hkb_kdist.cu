@@ -686,8 +686,8 @@ kdist_kernel(KdistArgs a) {
   const double inv = 1.0 / (double)nxb, iu = 1.0 / a.unitScale;
   for (int j = tid; j <= nxb / 2; j += THREADS) {
     const double x = grid_pos(j, (double)nxb, inv), x2 = 2.0 * x;
-    double ta = 1.0, tb = x, ev = 0.0, od = 0.0;
-    int i = 0;
+    double ta = __fma_rn(x2, x, -1.0), tb = __fma_rn(x2, ta, -x), ev = 0.0, od = 0.0;  // T_2, T_3
+    int i = 2;
     for (; i + 1 < nc; i += 2) {
       ev = __fma_rn(ta, s_c[i], ev);
       od = __fma_rn(tb, s_c[i + 1], od);
@@ -695,6 +695,10 @@ kdist_kernel(KdistArgs a) {
       tb = __fma_rn(x2, ta, -tb);
     }
     if (i < nc) ev = __fma_rn(ta, s_c[i], ev);
+    // the two largest terms last, so the others' roundings stay small (10000 x 20:
+    // 0.7e-15 rms of the value, 1.3e-15 with them first, 0.9e-15 by Clenshaw's sum)
+    ev += s_c[0];
+    if (nc > 1) od = __fma_rn(x, s_c[1], od);
     work[j] = exp(ev + od) * iu;
     if (j > 0 && nxb - j > j) work[nxb - j] = exp(ev - od) * iu;
   }
