@@ -196,6 +196,13 @@ static __host__ __device__ inline bool kdist_moments(int nxb, int nc) {
   return nc >= 4 && 6 * nc <= nxb && 2 * nc * nc <= 7 * nxb;
 }
 
+// Threads that sum a bin in the fit, by its size alone: the narrowest CTA that
+// holds it.  A wider CTA (few bins) lets as many of its threads sum in the same
+// order, so a state keeps its coefficients in any batch and on any GPU.
+static __host__ __device__ inline int kdist_sum_threads(int nxb) {
+  return nxb > 6144 ? KD_THREADS : nxb > 3072 ? KD_THREADS / 2 : KD_THREADS / 4;
+}
+
 struct KdistArgs {
   const double *K;       // nstates x nx, unsorted
   int64_t k_stride;
@@ -263,22 +270,25 @@ __device__ __forceinline__ double rescale_down(const double *work, int nxb, int 
   return __fma_rn(Kr - Kl, ii - il, Kl);
 }
 
-// leastSquare_kernel with the reflections: Q^T b by the first nc-1 of them,
-// thread tid owning the bin elements k = tid + n nt (k >= j) in every
-// reflection (one barrier each), then the back-substitution by one thread,
-// whose result is s_c (and co).  red: 64 doubles.
+// leastSquare_kernel with the reflections: Q^T b by the first nc-1 of them, the
+// sums by kdist_sum_threads threads, each its elements k = tid + n vt (k >= j) in
+// turn, then the back-substitution by one thread, whose result is s_c (and co).
+// A CTA of that width needs one barrier per reflection, a wider one another for
+// the elements that its other threads change.  red: 64 doubles.
 __device__ void fit_reflections(const KdistArgs &a, double *work, const double *s_cv, const double *s_d,
                                 double *red, double *s_c, double *__restrict__ co) {
-  const int nxb = a.nxb, nc = a.nc, tid = threadIdx.x, nt = blockDim.x;
+  const int nxb = a.nxb, nc = a.nc, tid = threadIdx.x, nt = blockDim.x, vt = kdist_sum_threads(nxb);
   for (int j = 0; j < nc - 1; ++j) {
     const double *vj = a.V + (int64_t)nxb * j;
     double dot = 0.0;
-    for (int k = tid; k < nxb; k += nt)
-      if (k >= j) dot = __fma_rn(vj[k], work[k], dot);
+    if (tid < vt)
+      for (int k = tid; k < nxb; k += vt)
+        if (k >= j) dot = __fma_rn(vj[k], work[k], dot);
     dot = block_sum1(dot, red, j & 1);
     const double t = dot / s_cv[j];
     for (int k = tid; k < nxb; k += nt)
       if (k >= j) work[k] = __fma_rn(-t, vj[k], work[k]);
+    if (nt > vt) __syncthreads();
   }
   __syncthreads();
   if (tid == 0) {
@@ -317,24 +327,28 @@ __device__ void fit_reflections(const KdistArgs &a, double *work, const double *
 // extended precision, median over spectra (reflections / moments of b / of
 // b - p): 10000 x 20 9.8e-16 / 2.8e-15 / 3.5e-16, 120 x 20 9.2e-16 / 3.2e-15 /
 // 3.8e-16, 2858 x 100 9.2e-16 / 9.1e-15 / 6.1e-16.
-// buf: (groups * KD_MG + 1) * warps doubles, then M if it fits.
+// The sums are those of VT = kdist_sum_threads threads of NF elements or more; a
+// wider CTA spreads their warps' groups over its own warps.
+// buf: (groups * KD_MG + 1) * VT / 32 doubles, then M if it fits.
 constexpr int KD_MG = 10;
-template <int THREADS, int IPT>
+template <int THREADS, int NF, int VT>
 __device__ __forceinline__ void fit_moments(const KdistArgs &a, const double *b, const double *s_d,
                                             double *buf, int buf_doubles, double *s_z,
                                             double *s_c, double *__restrict__ co) {
   constexpr int WARPS = THREADS / 32;
   const int n = a.nxb, nc = a.nc, nm = nc - 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int groups = (nm + KD_MG - 1) / KD_MG;
-  double *Ms = buf + (groups * KD_MG + 1) * WARPS;
-  const bool in_smem = (groups * KD_MG + 1) * WARPS + nc * nc <= buf_doubles;
+  constexpr int VW = VT / 32;
+  const bool sums = VT == THREADS || tid < VT;  // one of the VT threads
+  double *Ms = buf + (groups * KD_MG + 1) * VW;
+  const bool in_smem = (groups * KD_MG + 1) * VW + nc * nc <= buf_doubles;
   // M and f come from L2: their loads are issued before the moments' arithmetic
-  double f[IPT];
+  double f[NF];
   const double *ft = a.V + (int64_t)n * nm;  // f, rows >= nc - 1
 #pragma unroll
-  for (int i = 0; i < IPT; ++i) {
-    const int k = tid + i * THREADS;
-    f[i] = k < n ? (k < nm ? a.Cv[k] : ft[k]) : 0.0;
+  for (int i = 0; i < NF; ++i) {
+    const int k = tid + i * VT;
+    f[i] = sums && k < n ? (k < nm ? a.Cv[k] : ft[k]) : 0.0;
   }
   if (in_smem)
     for (int q = tid; q < nc * nc; q += THREADS) {
@@ -343,14 +357,15 @@ __device__ __forceinline__ void fit_moments(const KdistArgs &a, const double *b,
     }
   double af = 0.0;
 #pragma unroll
-  for (int i = 0; i < IPT; ++i) {
-    const int k = tid + i * THREADS;
-    if (k < n) af = __fma_rn(f[i], b[k], af);
+  for (int i = 0; i < NF; ++i) {
+    const int k = tid + i * VT;
+    if (sums && k < n) af = __fma_rn(f[i], b[k], af);
   }
   // (f is finite, but 0 x inf where b is not: the finite check below covers it)
-  for (int k = tid + IPT * THREADS; k < n; k += THREADS) af = __fma_rn(ft[k], b[k], af);
+  if (sums)
+    for (int k = tid + NF * VT; k < n; k += VT) af = __fma_rn(ft[k], b[k], af);
   for (int o = 16; o > 0; o >>= 1) af += __shfl_xor_sync(0xffffffffu, af, o);
-  if (lane == 0) buf[groups * KD_MG * WARPS + warp] = af;
+  if (lane == 0 && warp < VW) buf[groups * KD_MG * VW + warp] = af;
   // p = sum p_j T_j
   double p0, p1, p2, p3;
   {
@@ -362,20 +377,21 @@ __device__ __forceinline__ void fit_moments(const KdistArgs &a, const double *b,
     p3 = nc > 4 ? (de - 2.0 * di) * (1.0 / 6.0) : 0.0;
   }
   const double den = (double)n - 1.0, inv = 1.0 / den;
-  for (int gq = 0; gq < groups; ++gq) {
+  for (int u = warp; u < groups * VW; u += WARPS) {
+    const int gq = u / VW, w = VT == THREADS ? warp : u - gq * VW;  // group, and warp of the VT threads
     double acc[KD_MG];
 #pragma unroll
     for (int q = 0; q < KD_MG; ++q) acc[q] = 0.0;
-    for (int k = tid; k < (n + 1) / 2; k += THREADS) {
+    for (int k = w * 32 + lane; k < (n + 1) / 2; k += VT) {
       const int k2 = n - 1 - k;
       // (the middle point of an odd count has x = 0: odd T vanish)
       const bool two = k2 > k;
       const double bl = b[k], bh = two ? b[k2] : 0.0;
-      const double x = grid_pos(k, den, inv), x2 = 2.0 * x, w = two ? -2.0 : -1.0;
+      const double x = grid_pos(k, den, inv), x2 = 2.0 * x, m2 = two ? -2.0 : -1.0;
       double ta = __fma_rn(x2, x, -1.0), tb = __fma_rn(x2, ta, -x);  // T_2, T_3
       // sum and difference of b - p at x and -x
-      const double s = __fma_rn(w, __fma_rn(p2, ta, p0), bl + bh);
-      const double d = __fma_rn(w, __fma_rn(p3, tb, p1 * x), bl - bh);
+      const double s = __fma_rn(m2, __fma_rn(p2, ta, p0), bl + bh);
+      const double d = __fma_rn(m2, __fma_rn(p3, tb, p1 * x), bl - bh);
       if (gq == 0) {
         acc[0] += s;
         acc[1] = __fma_rn(x, d, acc[1]);
@@ -410,13 +426,13 @@ __device__ __forceinline__ void fit_moments(const KdistArgs &a, const double *b,
       for (int q = 0; q < KD_MG / 2; ++q) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
     if ((lane & 15) == 0)
 #pragma unroll
-      for (int q = 0; q < KD_MG / 2; ++q) buf[(gq * KD_MG + q + (up ? KD_MG / 2 : 0)) * WARPS + warp] = acc[q];
+      for (int q = 0; q < KD_MG / 2; ++q) buf[(gq * KD_MG + q + (up ? KD_MG / 2 : 0)) * VW + w] = acc[q];
   }
   __syncthreads();
   // sums over the warps: value v to s_z[v], f . b to s_z[nc - 1]
   for (int v = warp; v < nc; v += WARPS) {
     const int src = v < nm ? v : groups * KD_MG;
-    double t = lane < WARPS ? buf[src * WARPS + lane] : 0.0;
+    double t = lane < VW ? buf[src * VW + lane] : 0.0;
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     if (lane == 0) s_z[v] = t;
   }
@@ -567,7 +583,7 @@ __device__ __noinline__ void merge_sort(const double *__restrict__ src, int n, v
   __syncthreads();
 }
 
-// One CTA per (state, bin), THREADS IPT >= nxb points.
+// One CTA per (state, bin), THREADS IPT >= nxb points, VT = kdist_sum_threads(nxb).
 //
 // Sort: the keys' span in the bin (largest - smallest, in the order of the
 // FP64 bit patterns; points that no line reaches, at kmin, apart) is cut to
@@ -580,7 +596,7 @@ __device__ __noinline__ void merge_sort(const double *__restrict__ src, int n, v
 // Bound: latency, one 1024-thread CTA per SM in phases between barriers (load
 // 8 %, sort 35 %, ln 10 %, moments 25 %, reconstruction 16 % of a bin's time);
 // its 115 MB of traffic would take 18 us.
-template <int THREADS, int IPT>
+template <int THREADS, int IPT, int VT>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 kdist_kernel(KdistArgs a) {
   constexpr int WARPS = THREADS / 32;
@@ -676,7 +692,7 @@ kdist_kernel(KdistArgs a) {
   const int nc = a.nc;
   double *co = a.coeff + ((int64_t)s * a.nbins + b) * nc;
   if (kdist_moments(nxb, nc))
-    fit_moments<THREADS, IPT>(a, work, s_d, reinterpret_cast<double *>(cnt), KD_STEPS * THREADS / 2, s_z, s_c, co);
+    fit_moments<THREADS, IPT * (THREADS / VT) < 12 ? IPT * (THREADS / VT) : 12, VT>(a, work, s_d, reinterpret_cast<double *>(cnt), KD_STEPS * THREADS / 2, s_z, s_c, co);
   else
     fit_reflections(a, work, s_cv, s_d, red, s_c, co);
   if (a.recon == nullptr) return;
@@ -765,7 +781,7 @@ kdist_big_kernel(KdistArgs a) {
   __syncthreads();
   const int nc = a.nc;
   double *co = a.coeff + ((int64_t)s * a.nbins + b) * nc;
-  if (kdist_moments(nxb, nc)) fit_moments<KD_THREADS, 8>(a, work, s_d, s_buf, BUF, s_z, s_c, co);
+  if (kdist_moments(nxb, nc)) fit_moments<KD_THREADS, 8, KD_THREADS>(a, work, s_d, s_buf, BUF, s_z, s_c, co);
   else fit_reflections(a, work, s_cv, s_d, red, s_c, co);
   if (a.recon == nullptr) return;
 
@@ -860,27 +876,36 @@ cudaError_t launch_kdist(const double *K_d, int64_t k_stride, int nstates,
     kfn<<<grid, threads, dyn, stream>>>(a);
     return cudaGetLastError();
   };
-  // The smallest CTA that holds the bin at 12 keys a thread: 1024 threads
-  // share an SM, so the barriers of one bin hide behind another's work (20
+  // 1024 threads share an SM: the smallest CTA that holds the bin at 12 keys a
+  // thread lets the barriers of one bin hide behind another's work (20
   // coefficients, 3000 points: 3000 bins 191 us in 256 threads, 241 in 512, 346
-  // in 1024; 6000 points 395 in 512, 498 in 1024).  With fewer bins than SMs a
-  // wider one would finish sooner (3000 points 26 us in 512 against 31, 6000
-  // 33 in 1024 against 37), but the sums' order, and so the last bits of the
-  // coefficients, goes with the width: it depends on nxb alone, and a state
-  // keeps its coefficients whatever it is fitted with and wherever.
-  const int thr = nxb > 6144 ? 1024 : nxb > 3072 ? 512 : 256;
-  const int ipt = (nxb + thr - 1) / thr;
-#define KD_CASE(T, I) \
-  if (thr == T && ipt <= I) return run(kdist_kernel<T, I>, T, I);
-  KD_CASE(1024, 8)
-  KD_CASE(1024, 10)
-  KD_CASE(1024, 12)
-  KD_CASE(512, 8)
-  KD_CASE(512, 10)
-  KD_CASE(512, 12)
-  KD_CASE(256, 4)
-  KD_CASE(256, 8)
-  KD_CASE(256, 12)
+  // in 1024; 6000 points 395 in 512, 498 in 1024); with fewer bins than SMs a
+  // wider CTA finishes its bin sooner (30 bins of 3000 points 25 us in 1024
+  // threads, 31 in 256; 6000 points 33 in 1024, 37 in 512).  The coefficients
+  // are the same to the bit (kdist_sum_threads).
+  int dev = 0, nsm = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const int64_t ctas = (int64_t)nbins * nstates;
+  const int thr = (nxb > 6144 || ctas <= nsm) ? 1024 : (nxb > 3072 || ctas <= 2 * nsm) ? 512 : 256;
+  const int ipt = (nxb + thr - 1) / thr, vt = kdist_sum_threads(nxb);
+#define KD_CASE(T, I, V) \
+  if (thr == T && ipt <= I && vt == V) return run(kdist_kernel<T, I, V>, T, I);
+  KD_CASE(1024, 8, 1024)
+  KD_CASE(1024, 10, 1024)
+  KD_CASE(1024, 12, 1024)
+  KD_CASE(1024, 4, 512)
+  KD_CASE(1024, 6, 512)
+  KD_CASE(1024, 2, 256)
+  KD_CASE(1024, 4, 256)
+  KD_CASE(512, 8, 512)
+  KD_CASE(512, 10, 512)
+  KD_CASE(512, 12, 512)
+  KD_CASE(512, 4, 256)
+  KD_CASE(512, 8, 256)
+  KD_CASE(256, 4, 256)
+  KD_CASE(256, 8, 256)
+  KD_CASE(256, 12, 256)
 #undef KD_CASE
   return cudaErrorInvalidValue;
 }
